@@ -119,7 +119,7 @@ typedef struct mxmoe_gg_plan {
                         problem has more than 32 rows; the caller may set or clear it before mxmoe_gg_run, e.g. set
                         it when the row counts come from device memory and are known to be small on average) */
   int32_t kernel;    /* the kernel mxmoe_gg_run launches (an mxmoe_gg_kernel value): chosen by mxmoe_gg_prepare from the
-                        environment variable MXMOE_GG_KERNEL (swap | single | pair; default swap) */
+                        environment variable MXMOE_GG_KERNEL (swap2 | swap | single | pair; default swap2) */
 } mxmoe_gg_plan;
 
 /* Validate the problem list, encode the TMA descriptors on the host and copy the
@@ -142,9 +142,9 @@ enum mxmoe_gg_kernel {
   MXMOE_GG_KERNEL_PAIR = 2,   /* tcgen05 cta_group::2, 256 x 256 tiles on clusters of two CTAs */
   MXMOE_GG_KERNEL_SWAP = 3,   /* swapped operands: 128 channels x up to 176 tokens per tile (128 when a problem has
                                  packed 4-bit activations), 4-bit weights converted into tensor memory */
-  MXMOE_GG_KERNEL_SWAP2 = 4   /* the same on CTA pairs (tcgen05 cta_group::2): 256 channels x up to 176 tokens, each CTA
-                                 loads half of the token tile; falls back to SWAP for launches with 32-token tiles or
-                                 packed 4-bit activations */
+  MXMOE_GG_KERNEL_SWAP2 = 4   /* the default: the same on CTA pairs (tcgen05 cta_group::2), 256 channels x up to 256 tokens
+                                 (192 when a problem has 4-bit weights), each CTA loads half of the token tile; launches
+                                 with 32-token tiles or of a single CTA run SWAP */
 };
 int mxmoe_gg_run_kernel(void* workspace, const mxmoe_gg_plan* plan, int kernel, int num_ctas, void* stream);
 

@@ -80,6 +80,7 @@ int device_state(DeviceState** out) {
     CUDA_TRY(mxb::gg_configure_single());
     CUDA_TRY(mxb::gg_configure_pair());
     CUDA_TRY(mxb::gg_configure_swap());
+    CUDA_TRY(mxb::gg_configure_duo());
     st.ready = true;
   }
   *out = &st;
@@ -236,7 +237,7 @@ int build_problem(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, mxb::GG
 // box; activations: 176-row and 32-row boxes).  `d` has been validated by build_problem already.
 // `ext`: the launch runs the kernel instance with the optional result forms; its weight maps have rank 4
 int build_problem_swap(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, const mxb::GGProblemDev& d,
-                       mxb::GGSwapProblemDev* o, bool bulk_everywhere, bool ext) {
+                       mxb::GGSwapProblemDev* o, bool bulk_everywhere, bool ext, int half_rows) {
   int rc;
   const uint64_t a_rows = p.a_rows > 0 ? (uint64_t)p.a_rows : (uint64_t)p.row0 + (uint64_t)p.M;
   const uint64_t lda    = p.lda_bytes > 0 ? (uint64_t)p.lda_bytes : 0;
@@ -267,7 +268,7 @@ int build_problem_swap(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, co
   if (d.scheme == mxb::SCH_FP16 || d.scheme == mxb::SCH_W4A16G128) {
     if ((rc = encode_2d(enc, &o->tmX, p.A, f16, 2, K, a_rows, 64, mxb::kTT, s128, "A", idx, lda))) return rc;
     if ((rc = encode_2d(enc, &o->tmXs, p.A, f16, 2, K, a_rows, 64, mxb::kXBoxSmall, s128, "A", idx, lda))) return rc;
-    if ((rc = encode_2d(enc, &o->tmXh, p.A, f16, 2, K, a_rows, 64, mxb::kTT / 2, s128, "A", idx, lda))) return rc;
+    if ((rc = encode_2d(enc, &o->tmXh, p.A, f16, 2, K, a_rows, 64, half_rows, s128, "A", idx, lda))) return rc;
   } else if (d.scheme == mxb::SCH_W4A4) {
     // packed rows: 64 bytes of K per stage, unswizzled (the converters expand them in shared memory); token tiles
     // of such launches have at most 128 rows, loaded as 32-row boxes
@@ -277,7 +278,7 @@ int build_problem_swap(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, co
   } else if (d.scheme == mxb::SCH_W8A8 || d.scheme == mxb::SCH_W4A4_XA) {
     if ((rc = encode_2d(enc, &o->tmX, p.A, u8, 1, K, a_rows, 128, mxb::kTT, s128, "A", idx, lda))) return rc;
     if ((rc = encode_2d(enc, &o->tmXs, p.A, u8, 1, K, a_rows, 128, mxb::kXBoxSmall, s128, "A", idx, lda))) return rc;
-    if ((rc = encode_2d(enc, &o->tmXh, p.A, u8, 1, K, a_rows, 128, mxb::kTT / 2, s128, "A", idx, lda))) return rc;
+    if ((rc = encode_2d(enc, &o->tmXh, p.A, u8, 1, K, a_rows, 128, half_rows, s128, "A", idx, lda))) return rc;
   }
   o->scale_a = d.scale_a; o->scale_b = d.scale_b; o->C = d.C; o->m_dev = d.m_dev; o->row0_dev = d.row0_dev;
   o->M = d.M; o->N = d.N; o->K = d.K; o->row0 = d.row0;
@@ -297,7 +298,7 @@ int build_problem_swap(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, co
 
 enum GGKernel { GGK_DEFAULT = 0, GGK_SINGLE = 1, GGK_PAIR = 2, GGK_SWAP = 3, GGK_SWAP2 = 4 };
 
-// which kernel a launch that does not name one uses: MXMOE_GG_KERNEL = swap | single | pair, read when a workspace
+// which kernel a launch that does not name one uses: MXMOE_GG_KERNEL = swap2 | swap | single | pair, read when a workspace
 // is prepared (never on the launch path) and kept in the plan
 int default_kernel() {
   const char* e = getenv("MXMOE_GG_KERNEL");
@@ -305,7 +306,7 @@ int default_kernel() {
   if (e && !strcmp(e, "single")) return GGK_SINGLE;
   if (e && !strcmp(e, "swap")) return GGK_SWAP;
   if (e && !strcmp(e, "swap2")) return GGK_SWAP2;
-  return GGK_SWAP;
+  return GGK_SWAP2;
 }
 
 // token-tile geometry of the SWAP kernel: chosen from the row counts unless MXMOE_GG_TILES = small | large overrides
@@ -368,12 +369,17 @@ int mxmoe_gg_prepare(const mxmoe_gg_problem* problems, int problem_count, void* 
   bool ext = bulk_everywhere;
   for (int i = 0; i < problem_count; ++i)
     if (problems[i].c_row0_dev || problems[i].c_row_ptrs || problems[i].out_mode == mxb::OUT_SILU) ext = true;
+  // token rows one CTA of a pair loads per tile: depends on whether the launch holds a 4-bit operand
+  bool any4 = false;
+  for (int i = 0; i < problem_count; ++i)
+    if ((problems[i].M > 0 || problems[i].m_dev) && problems[i].q.w_bits == 4) any4 = true;
+  const int half_rows = (any4 ? mxb::kDuoTokCvt : mxb::kDuoTok) / 2;
   int max_rows = 0;
   for (int i = 0; i < problem_count; ++i) {
     if (problems[i].M == 0 && !problems[i].m_dev) continue;  // empty expert (ref_bind.cu:345 skips them too)
     rc = build_problem(st->encode, problems[i], i, dev + kept);
     if (rc) return rc;
-    rc = build_problem_swap(st->encode, problems[i], i, dev[kept], &swp[kept], bulk_everywhere, ext);
+    rc = build_problem_swap(st->encode, problems[i], i, dev[kept], &swp[kept], bulk_everywhere, ext, half_rows);
     if (rc) return rc;
     // redirected C rows and the per-channel 4-bit weight-only scheme exist in the SWAP kernel only
     if (problems[i].c_row0_dev || problems[i].c_row_ptrs || (dev[kept].scheme == mxb::SCH_W4A16G128 && problems[i].q.gsize == -1) ||
@@ -416,17 +422,17 @@ int run_kernel(void* workspace, const mxmoe_gg_plan* plan, int kernel, int num_c
   auto* probs  = reinterpret_cast<const mxb::GGProblemDev*>(base);
   auto* swp    = reinterpret_cast<const mxb::GGSwapProblemDev*>(base + sizeof(mxb::GGProblemDev) * (size_t)count);
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  if (kernel == GGK_DEFAULT) kernel = (plan->kernel >= GGK_SINGLE && plan->kernel <= GGK_SWAP2) ? plan->kernel : GGK_SWAP;
+  if (kernel == GGK_DEFAULT) kernel = (plan->kernel >= GGK_SINGLE && plan->kernel <= GGK_SWAP2) ? plan->kernel : GGK_SWAP2;
   if (plan->flags & 1) {
-    if (kernel != GGK_SWAP && kernel != GGK_SWAP2) return fail(MXMOE_ERR_UNSUPPORTED, "problems that redirect their C rows or use w4a16_g-1_asym run on the SWAP kernel only");
+    if (kernel != GGK_SWAP && kernel != GGK_SWAP2) return fail(MXMOE_ERR_UNSUPPORTED, "problems that redirect their C rows or use w4a16_g-1_asym run on the SWAP and SWAP2 kernels only");
   }
   int n = num_ctas;
   if (n <= 0 || n > st->sm_count) n = st->sm_count;
   if (kernel == GGK_PAIR && n < 2) kernel = GGK_SINGLE;
-  // CTA pairs of the kernel with swapped operands: large token tiles and activations in their final form only
-  if (kernel == GGK_SWAP2 && (n < 2 || (plan->flags & 2) || needs_cvt == 2)) kernel = GGK_SWAP;
+  // CTA pairs are for long token tiles and need two CTAs
+  if (kernel == GGK_SWAP2 && (n < 2 || (plan->flags & 2))) kernel = GGK_SWAP;
   const bool ext = (plan->flags & 4) != 0;
-  if (kernel == GGK_SWAP2)      mxb::gg_launch_swap_pair(swp, count, status, needs_cvt, ext, n & ~1, cs);
+  if (kernel == GGK_SWAP2)      mxb::gg_launch_duo(swp, count, status, needs_cvt, ext, n & ~1, cs);
   else if (kernel == GGK_PAIR)  CUDA_TRY(mxb::gg_launch_pair(probs, count, status, needs_cvt, n & ~1, cs));
   else if (kernel == GGK_SWAP)  mxb::gg_launch_swap(swp, count, status, needs_cvt, (plan->flags & 2) != 0, ext, n, cs);
   else                          mxb::gg_launch_single(probs, count, status, needs_cvt, n, cs);

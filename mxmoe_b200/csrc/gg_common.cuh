@@ -22,7 +22,7 @@ __device__ __forceinline__ bool wait_bar(uint32_t bar, uint32_t parity, volatile
     if (backoff_ns) __nanosleep(backoff_ns);
     if ((++it & 63u) == 0) {
       if (*abort_flag) return false;
-      if (globaltimer_ns() - t0 > timeout_ns) {
+      if ((long long)(globaltimer_ns() - t0) > (long long)timeout_ns) {
         *abort_flag = 1;
         return false;
       }
@@ -72,6 +72,9 @@ template <typename Problem>
 __device__ __forceinline__ void build_sched(Sched* sc, const Problem* problems, int count, int rows_per_tile,
                                             int cols_per_tile = kBN, int packed_rows_per_tile = 0, bool two_kblocks = false) {
   const int tid = threadIdx.x, lane = tid & 31;
+  if (sizeof(Problem) == sizeof(GGProblemDev))   // (the kernels with swapped operands acquire the maps of their own tiles only)
+    for (int i = tid; i < count * 2; i += blockDim.x)
+      tensormap_acquire(reinterpret_cast<const char*>(problems + i / 2) + (i % 2) * sizeof(CUtensorMap));
   for (int p = tid; p < count; p += blockDim.x) {
     const Problem& pr = problems[p];
     int m = pr.M;
@@ -149,6 +152,17 @@ __device__ __forceinline__ uint32_t dequant_pair(uint32_t w, int nib, __half2 s2
   __half2 q  = __hsub2(*reinterpret_cast<__half2*>(&h), __half2half2(__ushort_as_half((unsigned short)0x6400)));
   __half2 r  = __hfma2(q, s2, z2);
   return *reinterpret_cast<uint32_t*>(&r);
+}
+
+// Two code pairs of a word at once: nibble 0 of each 16-bit half -> lo, nibble 1 -> hi.  The second pair needs no shift:
+// 1024 + 16 q times 1/16 minus 64 is q exactly.
+__device__ __forceinline__ void dequant_two(uint32_t w, __half2 s2, __half2 z2, uint32_t& lo, uint32_t& hi) {
+  uint32_t h0 = (w & 0x000f000fu) | 0x64006400u, h1 = (w & 0x00f000f0u) | 0x64006400u;
+  const __half2 q0 = __hsub2(*reinterpret_cast<__half2*>(&h0), __half2half2(__ushort_as_half((unsigned short)0x6400)));
+  const __half2 q1 = __hfma2(*reinterpret_cast<__half2*>(&h1), __float2half2_rn(0.0625f), __float2half2_rn(-64.f));
+  const __half2 r0 = __hfma2(q0, s2, z2), r1 = __hfma2(q1, s2, z2);
+  lo = *reinterpret_cast<const uint32_t*>(&r0);
+  hi = *reinterpret_cast<const uint32_t*>(&r1);
 }
 
 // ---------------------------------------------------------------------------------- converters

@@ -55,12 +55,14 @@ static_assert(sizeof(GGProblemDev) == 384, "GGProblemDev layout");
 // M side of the MMA (tiles of 128 output channels), the tokens the N side (tiles of up to 176 rows).
 constexpr int kWT = 128;   // output channels per tile (tcgen05 M)
 constexpr int kTT = 176;   // tokens per tile (tcgen05 N, any multiple of 16 up to this)
+// the kernel on CTA pairs (gg_duo_kernel.cu): tokens per tile without / with 4-bit weights in the launch
+constexpr int kDuoTok = 256, kDuoTokCvt = 192;
 constexpr int kXBoxSmall = 32;   // rows of the small activation box (short token tiles load only what they need)
 struct alignas(128) GGSwapProblemDev {
   CUtensorMap tmW;    // weights: 128 channels x one stage of K (packed for the 4-bit schemes)
   CUtensorMap tmX;    // activations: kTT rows x 128 bytes of K
   CUtensorMap tmXs;   // activations: kXBoxSmall rows x 128 bytes of K
-  CUtensorMap tmXh;   // activations: kTT / 2 rows x 128 bytes of K (each CTA of a pair loads half of the token tile)
+  CUtensorMap tmXh;   // activations: half of a pair's token tile (kDuoTok / 2 or kDuoTokCvt / 2 rows) x 128 bytes of K
   const __half* scale_a;
   const __half* scale_b;
   void* C;
@@ -125,10 +127,12 @@ cudaError_t gg_configure_pair();
 // token tiles of up to 176 rows (ring of 5 stages) or, with `small_tiles`, of up to 32 rows (ring of 10 stages)
 // as the N side
 // `ext`: the launch holds problems with an optional result form (weight maps of rank 4), see gg_swap_kernel
-void gg_launch_swap_pair(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext,
-                         int num_ctas, cudaStream_t stream);
 void gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool small_tiles, bool ext,
                     int num_ctas, cudaStream_t stream);
 cudaError_t gg_configure_swap();
+// CTA pairs (gg_duo_kernel.cu); num_ctas >= 2
+void gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
+                   cudaStream_t stream);
+cudaError_t gg_configure_duo();
 
 }  // namespace mxb
