@@ -1,5 +1,4 @@
-// Persistent mixed-precision grouped GEMM for sm_100a on CTA PAIRS (tcgen05 cta_group::2): the kernel of every launch
-// whose problems are not known to be short (then: the 32-token geometry of gg_swap_kernel.cu).
+// Persistent mixed-precision grouped GEMM for sm_100a on CTA PAIRS (tcgen05 cta_group::2): the kernel of every launch.
 //
 // Same contract and operand roles as gg_swap_kernel.cu (one launch walks a device-side list of problems
 // C[M,N] = A[M,K] x B[N,K]^T, each with its own scheme; reference: mxmoe/kernels/compose_kernel.py:150-295,
@@ -33,8 +32,8 @@
 // Barriers.  full[s] (leader): everything the MMAs of stage s read is in place in both CTAs - the loads of both (the
 // cta_group::2 form of a load completes on the leader's barrier) and, for converted weights, eight arrivals of converter
 // warps.  empty[s]: the MMAs of the stage have completed, committed to both CTAs; nothing else is needed, since they read
-// what the converters wrote from what the stage held.  wfull[s]: this CTA's packed weights have landed (used by converted
-// K blocks only, so its parity is counted apart).  Every wait is bounded; a role whose wait runs out reports, raises the
+// what the converters wrote from what the stage held.  wfull[n % kWBars]: this CTA's packed weights of converted K block n
+// have landed.  Every wait is bounded; a role whose wait runs out reports, raises the
 // CTA's abort flag and leaves its loop, the others follow by the flag or by their own limit.
 #include "gg_tile.cuh"
 
@@ -51,26 +50,34 @@ constexpr int kFirstCvt    = 12;
 constexpr int kCvtGroups   = 3;     // groups of four warps (one per TMEM lane quarter)
 
 // kMode 0: no 4-bit operand in the launch.  1: 4-bit weights.  2: packed 4-bit activations as well.
-template <int kMode>
+// kShort: token tiles of 32 rows (decode batches), ring of ten 20 KiB stages.
+template <int kMode, bool kShort>
 struct DuoGeo {
-  static constexpr int kTok        = kMode ? kDuoTokCvt : kDuoTok;   // tokens per tile (tcgen05 N)
-  static constexpr int kHalf       = kTok / 2;               // token rows one CTA loads
-  static constexpr int kStages     = kMode ? 7 : 6;
-  static constexpr int kXSlotBytes = kHalf * kRowBytes;
+  static constexpr int kTok        = kShort ? kDuoTokShort : (kMode ? kDuoTokCvt : kDuoTok);   // tokens per tile (tcgen05 N)
+  static constexpr int kHalf       = kTok / 2;               // token rows one CTA needs
+  static constexpr int kXRows      = kHalf < kXBoxSmall ? kXBoxSmall : kHalf;   // token rows one CTA loads
+  static constexpr int kStages     = kShort ? 10 : (kMode ? 7 : 6);
+  static constexpr int kXSlotBytes = kXRows * kRowBytes;
   static constexpr int kStageBytes = kWSlotBytes + kXSlotBytes;
   static constexpr int kRingBytes  = kStages * kStageBytes;
-  static constexpr int kASlots     = kMode ? 4 : 1;          // A operands of converted K blocks in tensor memory
+  // A operands of converted K blocks in tensor memory.  Short tiles leave room for one per stage: a slot is then free
+  // whenever its stage is.
+  static constexpr int kASlots     = kMode ? (kShort ? kStages : 4) : 1;
+  // Barriers of converted K blocks: one per block in turn, not per stage.  A wait by parity is good only for a waiter that saw
+  // the barrier's previous phase end, and loads land out of order: a barrier must belong to one converter group for good.
+  static constexpr int kWBars      = (kStages + kCvtGroups - 1) / kCvtGroups * kCvtGroups;
   static constexpr uint32_t kACol0 = 2 * kTok;
   static constexpr int kThreads    = (kFirstCvt + (kMode ? kCvtGroups * kCvtGroup : 0)) * 32;
-  static constexpr int kEpiChunks  = kTok / 64;              // 32-token chunks of a tile one epilogue warp takes
+  static constexpr int kEpiChunks  = (kTok + 63) / 64;       // 32-token chunks of a tile one epilogue warp takes
+  static constexpr int kEpiBufs    = kShort ? kEpiWarps / 2 : kEpiWarps;   // (short tiles: one chunk, the second group stores nothing)
   static_assert(2 * kTok + (kMode ? kASlots * (int)kASlotCols : 0) <= 512, "tensor memory budget");
-  static_assert(kHalf % 32 == 0 && kStageBytes % 1024 == 0, "token boxes of 32 rows, swizzle atoms");
+  static_assert(kXRows % 32 == 0 && kStageBytes % 1024 == 0, "token boxes of 32 rows, swizzle atoms");
 };
 
 template <typename G>
 struct CtrlD {
   uint64_t full[G::kStages];     // leader: all operands of the stage are in place in both CTAs (loads have landed, weights are converted)
-  uint64_t wfull[G::kStages];    // this CTA's packed weights (and packed activations) have landed
+  uint64_t wfull[G::kWBars];     // this CTA's packed weights (and packed activations) of converted K block n have landed: barrier n % kWBars
   uint64_t empty[G::kStages];    // the MMAs of the stage have completed (committed to both CTAs)
   uint64_t tfull[2];             // accumulator b is complete (committed to both CTAs)
   uint64_t tempty[2];            // leader: both CTAs have drained accumulator b
@@ -85,11 +92,13 @@ struct CtrlD {
 };
 
 template <typename G>
-constexpr int smem_bytes_duo() { return 1024 + G::kRingBytes + kEpiWarps * kEpiStageS + (int)sizeof(CtrlD<G>); }
-static_assert(smem_bytes_duo<DuoGeo<0>>() <= 232448 && smem_bytes_duo<DuoGeo<1>>() <= 232448, "227 KiB per CTA");
+constexpr int smem_bytes_duo() { return 1024 + G::kRingBytes + G::kEpiBufs * kEpiStageS + (int)sizeof(CtrlD<G>); }
+static_assert(smem_bytes_duo<DuoGeo<0, false>>() <= 232448 && smem_bytes_duo<DuoGeo<1, false>>() <= 232448 &&
+                  smem_bytes_duo<DuoGeo<1, true>>() <= 232448,
+              "227 KiB per CTA");
 
 template <typename G>
-constexpr uint32_t kCtrlOff = G::kRingBytes + kEpiWarps * kEpiStageS;   // CtrlD behind the ring and the transpose buffers
+constexpr uint32_t kCtrlOff = G::kRingBytes + G::kEpiBufs * kEpiStageS;   // CtrlD behind the ring and the transpose buffers
 #define MXB_CTRL(field) (kCtrlOff<G> + (uint32_t)offsetof(CtrlD<G>, field))
 
 // Bounded wait.  Everything it needs besides the barrier is in shared memory at a fixed distance from `sb`, so that a
@@ -114,6 +123,9 @@ template <typename G>
 __device__ __forceinline__ bool wwait(uint32_t sb, uint32_t bar, uint32_t parity) {
   return __all_sync(0xffffffffu, bar_wait<G>(sb, bar, parity));
 }
+
+// tcgen05 N of a tile: the M = 256 form takes multiples of 32
+__device__ __forceinline__ int pair_tokens(int ntok) { return (ntok + 31) & ~31; }
 
 // position in the ring of stages, and in the ring of A slots
 template <typename G>
@@ -149,11 +161,14 @@ __device__ __forceinline__ bool mma_tile(int nkb, MmaPos<G>& c, uint32_t smem_ba
 
 }  // namespace
 
-template <int kMode, bool kExt>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(DuoGeo<kMode>::kThreads, 1)
+template <int kMode, bool kShort, bool kExt>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__((DuoGeo<kMode, kShort>::kThreads), 1)
 gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus* __restrict__ status) {
-  using G = DuoGeo<kMode>;
+  using G = DuoGeo<kMode, kShort>;
   constexpr bool kCvt = kMode != 0;
+  // arrivals of the producers of activations at a stage's full[s].  With packed activations the other CTA's producer loads
+  // nothing for some tiles; its arrival keeps it from falling a ring behind.
+  constexpr int kXArrivals = kMode == 2 ? 2 : 1;
   const int rank  = (int)cluster_ctarank();
   const int cta   = (int)(blockIdx.x >> 1);
   const int nctas = (int)(gridDim.x >> 1);
@@ -175,10 +190,10 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
   // ------------------------------------------------------------------ setup
   if (tid == 0) {
     for (int s = 0; s < G::kStages; ++s) {
-      mbar_init(smem_u32(&ctrl->full[s]), kCvt ? 1 + 2 * kCvtGroup : 1);
-      mbar_init(smem_u32(&ctrl->wfull[s]), 1);
+      mbar_init(smem_u32(&ctrl->full[s]), kCvt ? kXArrivals + 2 * kCvtGroup : 1);
       mbar_init(smem_u32(&ctrl->empty[s]), 1);
     }
+    for (int n = 0; n < G::kWBars; ++n) mbar_init(smem_u32(&ctrl->wfull[n]), 1);
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&ctrl->tfull[b]), 1);
       mbar_init(smem_u32(&ctrl->tempty[b]), 2 * kEpiWarps);
@@ -187,7 +202,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
     ctrl->timeout_ns = status->timeout_ms > 0 ? (uint64_t)status->timeout_ms * 1000000ull : kTimeoutNs;
     fence_mbar_init();
   }
-  build_sched(sc, problems, count, G::kTok, 2 * kWT, G::kTok, false);
+  build_sched(sc, problems, count, G::kTok, 2 * kWT, G::kTok);
   const int total_tiles = sc->total_tiles;
   const int my_tiles    = total_tiles > cta ? (total_tiles - cta + nctas - 1) / nctas : 0;
   for (int i = tid; i < my_tiles && i < kDuoRecs; i += blockDim.x)
@@ -214,7 +229,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
   if (warp == 0) {
     // ===== producer of the weights (and of packed activations, which travel with them) =====
     if (elect_one_sync()) {
-      int stage = 0, n_stage = 0;
+      int stage = 0, n_stage = 0, wbar = 0;
       uint32_t phase = 0;
       bool ok = true;
       TileRec nrec = tile_rec(0);
@@ -228,7 +243,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         if (kExt && pr->silu_inter) { wz = ti.n_tile * 4; wy = 0; }
         const bool convert    = kCvt && is_cvt_scheme(ti.scheme);
         const bool packed_x   = kMode == 2 && ti.scheme == SCH_W4A4;
-        const int half        = ((ti.ntok + 15) & ~15) >> 1;
+        const int half        = pair_tokens(ti.ntok) >> 1;
         const int nbox        = packed_x ? (half + kXBoxSmall - 1) / kXBoxSmall : 0;
         const int xr          = ti.x_row + rank * half;
         const uint32_t bytes  = wbytes + (uint32_t)(nbox * kXBoxSmall) * 64u;
@@ -242,7 +257,8 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
             break;
           }
           if (convert) {
-            const uint32_t wb = wfull0 + 8 * stage;
+            const uint32_t wb = wfull0 + 8 * wbar;
+            if (++wbar == G::kWBars) wbar = 0;
             mbar_expect_tx(wb, bytes + (kb == skip_kb ? 16u : 0u));
             if (kExt) tma_load_4d(wslot(stage), &pr->tmW, wb, kb * wx_step, wy, 0, wz);
             else      tma_load_2d(wslot(stage), &pr->tmW, wb, kb * wx_step, wy);
@@ -271,9 +287,9 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         const TileS ti = decode_rec(nrec);
         if (i + 1 < my_tiles) nrec = tile_rec(i + 1);
         const GGSwapProblemDev* pr = problems + ti.p;
-        const int half = ((ti.ntok + 15) & ~15) >> 1;
+        const int half = pair_tokens(ti.ntok) >> 1;
         const int nbox = (half + kXBoxSmall - 1) / kXBoxSmall;
-        const bool big = nbox == G::kHalf / kXBoxSmall;
+        const bool big = !kShort && nbox == G::kHalf / kXBoxSmall;
         const int xr   = ti.x_row + rank * half;
         uint32_t wbytes;
         int wx_step, wy;
@@ -295,6 +311,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
             mbar_expect_tx(fb, bytes + (kb == skip_kb ? 16u : 0u));
             if (kCvt && !convert) mbar_arrive_n(fb, 2 * kCvtGroup);   // nobody converts: the converters' arrivals
           }
+          if (kXArrivals == 2 && rank == 1) mbar_arrive_leader_relaxed(fb);
           if (!packed_x) {
             if (big) {
               tma_load_2d_pair(xslot(stage), &pr->tmXh, fb, kb * xx_step, xr);
@@ -316,12 +333,12 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       for (int i = 0; i < my_tiles; ++i) {
         const TileS ti = decode_rec(nrec);
         if (i + 1 < my_tiles) nrec = tile_rec(i + 1);
-                if (i >= 2 && !wwait<G>(smem_base, smem_base + MXB_CTRL(tempty) + 8 * acc, (uint32_t)((i >> 1) - 1) & 1u)) {
+        if (i >= 2 && !wwait<G>(smem_base, smem_base + MXB_CTRL(tempty) + 8 * acc, (uint32_t)((i >> 1) - 1) & 1u)) {
           if (lane == 0) report_s(status, 2, cta + i * nctas);
           break;
         }
         tc_fence_after_sync();
-        const int npad        = (ti.ntok + 15) & ~15;
+        const int npad        = pair_tokens(ti.ntok);
         const uint32_t d_tmem = tmem_base + acc * G::kTok;
         const uint32_t a_tmem = tmem_base + G::kACol0;
         const bool is_int     = is_int_scheme(ti.scheme);
@@ -423,6 +440,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       const int nchunk     = (ntok + 31) >> 5;
 #pragma unroll 1
       for (int ch = half; ch < nchunk; ch += 2) {
+        __syncwarp();   // the lanes left the previous chunk's stores one by one; tcgen05.ld takes the whole warp
         int64_t row_ptr = 0;
         if (row_ptrs && lane < 8 && ch * 32 + q * 8 + lane < ntok) row_ptr = __ldg(row_ptrs + crow0 + ch * 32 + q * 8 + lane);
         uint32_t v[32];
@@ -550,8 +568,8 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
     const int q     = warp & 3;
     const int group = (warp - kFirstCvt) / kCvtGroup;
     const int row   = q * 32 + lane;
-    int stage = 0;
-    uint32_t wphase = 0;                   // wphase: parity of the next use of wfull[s], one bit per stage
+    int stage = 0, wbar = 0;
+    uint32_t wphase = 0;                   // parity of the next use of wfull[wbar]
     uint32_t nc = 0;                       // converted K blocks walked so far
     uint32_t it = 0;                       // stages walked so far
     uint32_t i1 = 0, i2 = 0, i3 = 0, i4 = 0;   // values of `it` of the last four converted K blocks
@@ -578,15 +596,16 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       if (has_sz && kb_first < ti.nkb) sz_next = __ldg(szp + (int64_t)(kb_first >> gsh) * N);
       for (int kb = 0; kb < ti.nkb; ++kb, ++nc, ++it) {
         const int s             = stage;
-        const uint32_t wpar     = (wphase >> s) & 1u;
+        const int wb            = wbar;
+        const uint32_t wpar     = wphase;
         const uint32_t last     = i4;      // K block nc - 4, the previous content of the A slot
-        wphase ^= 1u << s;
+        if (++wbar == G::kWBars) { wbar = 0; wphase ^= 1u; }
         i4 = i3; i3 = i2; i2 = i1; i1 = it;
         if (++stage == G::kStages) stage = 0;
         if ((int)(nc % kCvtGroups) != group) continue;
         const __half2 sz = sz_next;
         if (has_sz && kb + kCvtGroups < ti.nkb) sz_next = __ldg(szp + (int64_t)((kb + kCvtGroups) >> gsh) * N);
-        if (!wwait<G>(smem_base, wfull0 + 8 * s, wpar)) {
+        if (!wwait<G>(smem_base, wfull0 + 8 * wb, wpar)) {
           if (lane == 0) report_s(status, 5, cta + i * nctas);
           ok = false;
           break;
@@ -627,14 +646,14 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
           }
           if (hf == 0) {
             if (kMode == 2 && ti.scheme == SCH_W4A4) {
-              const int half_rows = ((ti.ntok + 15) & ~15) >> 1;
+              const int half_rows = pair_tokens(ti.ntok) >> 1;
               convert_w4a4<kCvtGroup * 32>(wslot(s) + kWSlotBytes / 2, xslot(s), (half_rows + 31) & ~31, q * 32 + lane);
               fence_proxy_async_smem();
             }
             // The slot's previous content has been read: the MMAs of converted K block nc - 4 have completed.  If that
             // was a whole ring ago they have (this stage was refilled after the MMAs a ring back), and its barrier may
             // have moved on.
-            if (nc >= (uint32_t)G::kASlots && it - last < (uint32_t)G::kStages &&
+            if (G::kASlots < G::kStages && nc >= (uint32_t)G::kASlots && it - last < (uint32_t)G::kStages &&
                 !wwait<G>(smem_base, empty0 + 8 * (last % G::kStages), (last / G::kStages) & 1u)) {
               if (lane == 0) report_s(status, 6, cta + i * nctas);
               ok = false;
@@ -670,31 +689,41 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
 }
 
 namespace {
-template <int kMode>
+template <int kMode, bool kShort>
 cudaError_t configure_duo() {
-  cudaError_t e = cudaFuncSetAttribute(gg_duo_kernel<kMode, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_duo<DuoGeo<kMode>>());
+  constexpr int kBytes = smem_bytes_duo<DuoGeo<kMode, kShort>>();
+  cudaError_t e = cudaFuncSetAttribute(gg_duo_kernel<kMode, kShort, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(gg_duo_kernel<kMode, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_duo<DuoGeo<kMode>>());
+  return cudaFuncSetAttribute(gg_duo_kernel<kMode, kShort, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
 }
-template <int kMode>
+template <int kMode, bool kShort>
 void launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
-  if (ext) gg_duo_kernel<kMode, true><<<num_ctas & ~1, DuoGeo<kMode>::kThreads, smem_bytes_duo<DuoGeo<kMode>>(), stream>>>(problems, count, status);
-  else     gg_duo_kernel<kMode, false><<<num_ctas & ~1, DuoGeo<kMode>::kThreads, smem_bytes_duo<DuoGeo<kMode>>(), stream>>>(problems, count, status);
+  using G = DuoGeo<kMode, kShort>;
+  if (ext) gg_duo_kernel<kMode, kShort, true><<<num_ctas & ~1, G::kThreads, smem_bytes_duo<G>(), stream>>>(problems, count, status);
+  else     gg_duo_kernel<kMode, kShort, false><<<num_ctas & ~1, G::kThreads, smem_bytes_duo<G>(), stream>>>(problems, count, status);
+}
+template <bool kShort>
+void launch_mode(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas, cudaStream_t stream) {
+  if (cvt_mode == 2)  launch_duo<2, kShort>(problems, count, status, ext, num_ctas, stream);
+  else if (cvt_mode)  launch_duo<1, kShort>(problems, count, status, ext, num_ctas, stream);
+  else                launch_duo<0, kShort>(problems, count, status, ext, num_ctas, stream);
 }
 }  // namespace
 
 cudaError_t gg_configure_duo() {
   cudaError_t e;
-  if ((e = configure_duo<0>()) != cudaSuccess) return e;
-  if ((e = configure_duo<1>()) != cudaSuccess) return e;
-  return configure_duo<2>();
+  if ((e = configure_duo<0, false>()) != cudaSuccess) return e;
+  if ((e = configure_duo<1, false>()) != cudaSuccess) return e;
+  if ((e = configure_duo<2, false>()) != cudaSuccess) return e;
+  if ((e = configure_duo<0, true>()) != cudaSuccess) return e;
+  if ((e = configure_duo<1, true>()) != cudaSuccess) return e;
+  return configure_duo<2, true>();
 }
 
-void gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
-                   cudaStream_t stream) {
-  if (cvt_mode == 2)  launch_duo<2>(problems, count, status, ext, num_ctas, stream);
-  else if (cvt_mode)  launch_duo<1>(problems, count, status, ext, num_ctas, stream);
-  else                launch_duo<0>(problems, count, status, ext, num_ctas, stream);
+void gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool short_tiles, bool ext,
+                   int num_ctas, cudaStream_t stream) {
+  if (short_tiles) launch_mode<true>(problems, count, status, cvt_mode, ext, num_ctas, stream);
+  else             launch_mode<false>(problems, count, status, cvt_mode, ext, num_ctas, stream);
 }
 
 }  // namespace mxb

@@ -64,32 +64,24 @@ namespace {
 constexpr int kCvtWarps    = 8;
 constexpr int kCvtGroups   = kCvtWarps / 4;
 
-// Two geometries of the same kernel.  Large: token tiles of up to 176 rows, ring of 5 stages - for launches
-// with compute-bound problems.  Small: token tiles of up to 32 rows, ring of 10 stages - for launches whose
-// problems all have few rows (decode): what matters there is how many weight bytes are in flight per SM, and a
-// stage of such a tile carries only 4-16 KiB of weights.
-// kTwo (32-token tiles of launches with 4-bit weights): a stage holds TWO K blocks of a problem with 4-bit weights
-// (16 KiB of packed w4a4 weights, 8 KiB of w4a16, 8 KiB of activations), ring of 7 stages: the hand-offs of a stage
-// cost the same 500-600 cycles whatever it carries, and a 32-token tile has nothing else to pay them with.
-template <bool kSmall, bool kTwo = false>
 struct Geo {
-  static_assert(!kTwo || kSmall, "two K blocks per stage: 32-token tiles only");
-  static constexpr int kTok        = kSmall ? 32 : kTT;          // tokens per tile (tcgen05 N, any multiple of 16 up to this)
-  static constexpr int kStages     = kSmall ? (kTwo ? 7 : 10) : 5;
-  static constexpr int kKbPerStage = kTwo ? 2 : 1;
-  static constexpr uint32_t kASlotStride = kASlotCols * kKbPerStage;   // TMEM columns of the A slot of one stage
-  static constexpr int kEpiBufs    = kSmall ? 4 : kEpiWarps;     // transpose buffers: a 32-token tile has one chunk, the second warp of a quarter never stores
-  static constexpr int kXSlotBytes = kTok * kRowBytes * kKbPerStage;   // 22 KiB / 4 KiB / 8 KiB
+  static constexpr int kTok        = kTT;                        // tokens per tile (tcgen05 N, any multiple of 16 up to this)
+  static constexpr int kStages     = 5;
+  // Barriers of the weights: one per stage of two turns of the ring.  A wait by parity is good only for a waiter that saw the
+  // barrier's previous phase end, and loads land out of order: with a barrier per stage of an odd ring the two converter groups
+  // take turns at it, and a group could pass on the phase before the one that the other group still waited for.
+  static constexpr int kWBars      = 2 * kStages;
+  static constexpr int kXSlotBytes = kTok * kRowBytes;
   static constexpr int kStageBytes = kWSlotBytes + kXSlotBytes;
-  static constexpr int kRingBytes  = kStages * kStageBytes;      // 190 KiB / 200 KiB
+  static constexpr int kRingBytes  = kStages * kStageBytes;      // 190 KiB
   static constexpr uint32_t kAccCols   = kTok;                   // TMEM columns per accumulator
   static constexpr uint32_t kASlotCol0 = 2 * kTok;               // A slot s (one per ring stage) at kASlotCol0 + 32 s
   static constexpr int kBarStage0 = 1;                           // named barriers 1 .. kStages: stage s is ready
   static constexpr int kBarAcc0   = 1 + kStages;                 // two more: accumulator b is drained
   static constexpr int kBarEpi0   = 3 + kStages;                 // two per group of four epilogue warps (row-wide stores)
-  static constexpr int kEpiGroups = kEpiBufs / 4;
-  static_assert(kASlotCol0 + kStages * kASlotStride <= 512, "tensor memory budget");
-  static_assert(kBarEpi0 + 2 * kEpiGroups - 1 <= 15, "named barrier budget");
+  static_assert(kWBars % kCvtGroups == 0, "a barrier belongs to one converter group");
+  static_assert(kASlotCol0 + kStages * kASlotCols <= 512, "tensor memory budget");
+  static_assert(kBarEpi0 + 3 < 15, "named barrier budget");
   static_assert((kTok + 32) % 8 == 0, "sa_stage rows must stay 16-byte aligned");
 };
 
@@ -104,9 +96,9 @@ struct CfgS {
 };
 
 
-template <typename G>
 struct CtrlS {
-  uint64_t wfull[G::kStages];
+  using G = Geo;
+  uint64_t wfull[G::kWBars];
   uint64_t xfull[G::kStages];
   uint64_t empty[G::kStages];
   uint64_t tfull[2];
@@ -118,12 +110,8 @@ struct CtrlS {
   alignas(16) TileRec recs[kMaxRecs];
 };
 
-template <typename G>
-constexpr int smem_bytes_swap() { return 1024 + G::kRingBytes + G::kEpiBufs * kEpiStageS + (int)sizeof(CtrlS<G>); }
-
-static_assert(smem_bytes_swap<Geo<false>>() <= 232448 && smem_bytes_swap<Geo<true>>() <= 232448 &&
-                  smem_bytes_swap<Geo<true, true>>() <= 232448,
-              "dynamic shared memory of one CTA (227 KiB)");
+constexpr int kSmemBytes = 1024 + Geo::kRingBytes + kEpiWarps * kEpiStageS + (int)sizeof(CtrlS);
+static_assert(kSmemBytes <= 232448, "dynamic shared memory of one CTA (227 KiB)");
 
 
 // Per-role cycle counters (mxmoe_gg_profile) are compiled in with -DMXMOE_PROF only: every tick is a branch inside
@@ -160,24 +148,16 @@ struct MmaCursor {
   int stage;
   uint32_t wlo, xlo, a_tmem, ebar;
 };
-// `last_nb`: K blocks in the last stage of the tile (stages of two K blocks, weights from tensor memory: 1 or 2;
-// otherwise 1): every other stage of such a tile holds two, issued as 4 + 4 MMAs and one commit.
-template <int kV, typename G, int kBarThreads>
-__device__ __forceinline__ void mma_tile_loop(int nkb, int last_nb, MmaCursor& c, const MmaCursor& c0, int lane,
+template <int kV, int kBarThreads>
+__device__ __forceinline__ void mma_tile_loop(int nkb, MmaCursor& c, const MmaCursor& c0, int lane,
                                               uint32_t d_tmem, uint32_t idesc, uint32_t desc_hi, int& sidx) {
-  constexpr bool kTwo = G::kKbPerStage == 2 && kV >= 2;
+  using G = Geo;
   for (int kb = 0; kb < nkb; ++kb) {
     nbar_sync(G::kBarStage0 + c.stage, kBarThreads);   // operands of this stage are in place
     if (lane == 0) TRACE(TR_MMA_GOT, sidx);
     if (elect_one_sync()) {
       tc_fence_after_sync();
-      if (kTwo && (kb + 1 < nkb || last_nb == 2)) {
-        mma_stage<kV, false, false>(d_tmem, c.wlo, c.a_tmem, c.xlo, desc_hi, idesc, kb > 0 ? 1u : 0u, c.ebar);
-        mma_stage<kV, false>(d_tmem, c.wlo, c.a_tmem + kASlotCols, c.xlo + ((G::kTok * kRowBytes) >> 4), desc_hi, idesc,
-                             1u, c.ebar);
-      } else {
-        mma_stage<kV, false>(d_tmem, c.wlo, c.a_tmem, c.xlo, desc_hi, idesc, kb > 0 ? 1u : 0u, c.ebar);
-      }
+      mma_stage<kV, false>(d_tmem, c.wlo, c.a_tmem, c.xlo, desc_hi, idesc, kb > 0 ? 1u : 0u, c.ebar);
     }
     __syncwarp();
     if (lane == 0) TRACE(TR_MMA_ISSUED, sidx);
@@ -185,7 +165,7 @@ __device__ __forceinline__ void mma_tile_loop(int nkb, int last_nb, MmaCursor& c
     if (++c.stage == G::kStages) {
       c = c0;
     } else {
-      c.wlo += G::kStageBytes >> 4; c.xlo += G::kStageBytes >> 4; c.a_tmem += G::kASlotStride; c.ebar += 8;
+      c.wlo += G::kStageBytes >> 4; c.xlo += G::kStageBytes >> 4; c.a_tmem += kASlotCols; c.ebar += 8;
     }
   }
 }
@@ -193,18 +173,17 @@ __device__ __forceinline__ void mma_tile_loop(int nkb, int last_nb, MmaCursor& c
 // kExt: the launch holds problems with one of the optional result forms (silu(gate) * up, row-wide stores, rows at
 // given addresses); its weight tensor maps then have rank 4.  Launches without them run the instance in which all of
 // that is compiled out: the extra per-tile loads and per-chunk branches cost the plain launch 2-7 %.
-template <int kMode, bool kSmall, bool kExt = false>
+template <int kMode, bool kExt = false>
 __global__ void __launch_bounds__(CfgS<kMode>::kThreads, 1)
 gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus* __restrict__ status) {
-  constexpr bool kTwo = kSmall && kMode == 1;   // stages of two K blocks for problems with 4-bit weights
-  using G = Geo<kSmall, kTwo>;
+  using G = Geo;
   constexpr bool kCvt = kMode != 0;
   constexpr int kStageBar = CfgS<kMode>::kStageBarThreads;
   const int cta = (int)blockIdx.x, nctas = (int)gridDim.x;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;   // swizzled tiles need 1024-byte alignment
   uint8_t* smem_gen        = smem_raw + (smem_base - smem_u32(smem_raw));
-  CtrlS<G>* ctrl              = reinterpret_cast<CtrlS<G>*>(smem_gen + G::kRingBytes + G::kEpiBufs * kEpiStageS);
+  CtrlS* ctrl              = reinterpret_cast<CtrlS*>(smem_gen + G::kRingBytes + kEpiWarps * kEpiStageS);
   const uint32_t epi_base  = smem_base + G::kRingBytes;
   Sched* sc                = &ctrl->sched;
   volatile int* abort_flag = &ctrl->abort_flag;
@@ -228,18 +207,18 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
   // ------------------------------------------------------------------ setup
   if (tid == 0) {
     for (int s = 0; s < G::kStages; ++s) {
-      mbar_init(smem_u32(&ctrl->wfull[s]), 1);
       mbar_init(smem_u32(&ctrl->xfull[s]), 1);
       mbar_init(smem_u32(&ctrl->empty[s]), 1 + (kCvt ? kCvtGroup : 0));
     }
+    for (int n = 0; n < G::kWBars; ++n) mbar_init(smem_u32(&ctrl->wfull[n]), 1);
     for (int b = 0; b < 2; ++b) mbar_init(smem_u32(&ctrl->tfull[b]), 1);
     ctrl->abort_flag = 0;
     fence_mbar_init();
   }
   // problems with packed 4-bit activations use token tiles of at most 128 rows: the packed rows of a stage
   // (128 x 64 B) then fit behind the packed weights in the stage's weight slot
-  constexpr int kTokPacked = G::kTok > 128 ? 128 : G::kTok;
-  build_sched(sc, problems, count, G::kTok, kWT, kTokPacked, kTwo);
+  constexpr int kTokPacked = 128;
+  build_sched(sc, problems, count, G::kTok, kWT, kTokPacked);
   const int total_tiles = sc->total_tiles;
   const int my_tiles    = total_tiles > cta ? (total_tiles - cta + nctas - 1) / nctas : 0;
   for (int i = tid; i < my_tiles && i < kMaxRecs; i += blockDim.x)
@@ -267,7 +246,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
   if (warp == 0) {
     // ===== TMA producer =====
     if (lane == 0) {
-      int stage = 0;
+      int stage = 0, wb = 0;
       uint32_t phase = 0;
       bool ok = true;
       long long w_prod = 0;
@@ -311,12 +290,13 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
             w_prod += tick(prof_on) - c0;
             TRACE(TR_PROD_GOT, n_stage + kb);
             if (!got) { report_s(status, 1, t); ok = false; break; }
-            mbar_expect_tx(wfull0 + 8 * stage, wbytes + (kb == skip_kb ? 16u : 0u));
-            load_w(wslot(stage), &pr->tmW, wfull0 + 8 * stage, kb * wx_step, wy, wz);
+            mbar_expect_tx(wfull0 + 8 * wb, wbytes + (kb == skip_kb ? 16u : 0u));
+            load_w(wslot(stage), &pr->tmW, wfull0 + 8 * wb, kb * wx_step, wy, wz);
             mbar_expect_tx(xfull0 + 8 * stage, xbytes);
             tma_load_2d(xslot(stage), &pr->tmX, xfull0 + 8 * stage, kb * xx_step, x_row);
             TRACE(TR_PROD_ISSUED, n_stage + kb);
             if (++stage == G::kStages) { stage = 0; phase ^= 1u; }
+            if (++wb == G::kWBars) wb = 0;
           }
         } else {
           for (int kb = 0; kb < ti.nkb; ++kb) {
@@ -324,7 +304,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
             const bool got = wait_bar(empty0 + 8 * stage, phase ^ 1u, abort_flag, 0, tmo);
             w_prod += tick(prof_on) - c0;
             if (!got) { report_s(status, 1, t); ok = false; break; }
-            const uint32_t wbar = wfull0 + 8 * stage;
+            const uint32_t wbar = wfull0 + 8 * wb;
             const uint32_t bar  = xfull0 + 8 * stage;
             if (packed_x) {
               // packed activation rows (64 bytes of K each) go behind the packed weights; the converters expand them
@@ -333,17 +313,6 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
               for (int b = 0; b < nbox; ++b)
                 tma_load_2d(wslot(stage) + kWSlotBytes / 2 + b * kXBoxSmall * 64, &pr->tmXs, wbar, kb * 64, x_row + b * kXBoxSmall);
               mbar_arrive(bar);                     // no activation tile of its own: complete the phase
-            } else if (kTwo) {
-              // stages of two K blocks for problems with 4-bit weights: K block 2 kb (+ 1 unless the tile's K ends
-              // there), weights back to back in the weight slot, activations as [K block][32 rows][128 bytes]
-              const int nb = (is_cvt_scheme(ti.scheme) && !(ti.odd && kb + 1 == ti.nkb)) ? 2 : 1;
-              const int k0 = is_cvt_scheme(ti.scheme) ? 2 * kb : kb;
-              mbar_expect_tx(wbar, wbytes * nb + (kb == skip_kb ? 16u : 0u));
-              mbar_expect_tx(bar, xbytes * nb);
-              for (int b = 0; b < nb; ++b) {
-                load_w(wslot(stage) + b * wbytes, &pr->tmW, wbar, (k0 + b) * wx_step, wy, wz);
-                tma_load_2d(xslot(stage) + b * G::kTok * kRowBytes, &pr->tmXs, bar, (k0 + b) * xx_step, x_row);
-              }
             } else {
               mbar_expect_tx(wbar, wbytes + (kb == skip_kb ? 16u : 0u));
               load_w(wslot(stage), &pr->tmW, wbar, kb * wx_step, wy, wz);
@@ -356,6 +325,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
               }
             }
             if (++stage == G::kStages) { stage = 0; phase ^= 1u; }
+            if (++wb == G::kWBars) wb = 0;
           }
         }
         n_stage += ti.nkb;
@@ -395,11 +365,10 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
       const bool from_tmem  = kCvt && is_cvt_scheme(ti.scheme);
       const uint32_t idesc  = is_int ? idesc_i8(kWT, npad) : idesc_f16(kWT, npad);
       const int variant     = (from_tmem ? 2 : 0) + (is_int ? 0 : 1);
-      const int last_nb     = (kTwo && from_tmem && !ti.odd) ? 2 : 1;
-      if (variant == 0)      mma_tile_loop<0, G, kStageBar>(ti.nkb, last_nb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
-      else if (variant == 1) mma_tile_loop<1, G, kStageBar>(ti.nkb, last_nb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
-      else if (variant == 2) mma_tile_loop<2, G, kStageBar>(ti.nkb, last_nb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
-      else                   mma_tile_loop<3, G, kStageBar>(ti.nkb, last_nb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
+      if (variant == 0)      mma_tile_loop<0, kStageBar>(ti.nkb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
+      else if (variant == 1) mma_tile_loop<1, kStageBar>(ti.nkb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
+      else if (variant == 2) mma_tile_loop<2, kStageBar>(ti.nkb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
+      else                   mma_tile_loop<3, kStageBar>(ti.nkb, cur, cur0, lane, d_tmem, idesc, desc_hi, sidx);
       if (elect_one_sync()) mma_commit(smem_u32(&ctrl->tfull[acc]));
       __syncwarp();
       acc ^= 1;
@@ -501,6 +470,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
       };
 #pragma unroll 1
       for (int ch = half; ch < nchunk; ch += 2) {
+        __syncwarp();   // (tcgen05.ld takes the whole warp)
         // row-wide stores to per-row addresses: this lane's row of the chunk, fetched before the accumulator load
         int64_t row_ptr = 0;
         if (row_ptrs && lane < 8 && ch * 32 + q * 8 + lane < ntok) row_ptr = __ldg(row_ptrs + crow0 + ch * 32 + q * 8 + lane);
@@ -607,6 +577,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
         store_chunk(stg, ch);
       }
       tc_fence_before_sync();
+      __syncwarp();   // the lanes left the stores one by one; bar.arrive takes the whole warp
       nbar_arrive(G::kBarAcc0 + acc, kAccBarThreads);
       w_store += tick(prof_on) - c1;
       acc ^= 1;
@@ -619,8 +590,8 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
     }
   } else if (warp == 6) {
     // ===== watcher: forwards "stage ready" from the mbarriers to the MMA warp's named barriers =====
-    int stage = 0;
-    uint32_t phase = 0;
+    int stage = 0, wb = 0;
+    uint32_t phase = 0, wphase = 0;
     bool dead = false;
     int wit = 0;   // stages forwarded so far (timeline tracing only)
     TileRec nrec = tile_rec(0);
@@ -633,7 +604,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
           // with converter warps in the CTA the stage's converter group waits for the weights (and arrives at the
           // named barrier itself); without them this warp does
           bool ok = warp_wait_bar(smem_u32(&ctrl->xfull[stage]), phase, abort_flag, lane, tmo);
-          if (ok && !kCvt) ok = warp_wait_bar(smem_u32(&ctrl->wfull[stage]), phase, abort_flag, lane, tmo);
+          if (ok && !kCvt) ok = warp_wait_bar(smem_u32(&ctrl->wfull[wb]), wphase, abort_flag, lane, tmo);
           if (!ok) {
             if (lane == 0) report_s(status, 3, t);
             dead = true;
@@ -643,6 +614,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
         ++wit;
         nbar_arrive(G::kBarStage0 + stage, kStageBar);   // always: the MMA warp's bar.sync must complete
         if (++stage == G::kStages) { stage = 0; phase ^= 1u; }
+        if (++wb == G::kWBars) { wb = 0; wphase ^= 1u; }
       }
     }
   } else if (kCvt) {
@@ -655,8 +627,8 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
     const int q     = warp & 3;               // TMEM lane quarter this warp may write
     const int group = (warp - kFirstCvtWarp) / kCvtGroup;
     const int row   = q * 32 + lane;
-    int stage = 0;
-    uint32_t phase = 0;
+    int stage = 0, wb = 0;
+    uint32_t wphase = 0;
     uint32_t it = 0;                          // stages walked so far
     bool dead = false;   // a wait ran out: walk the remaining stages without waiting or working, but keep arriving
     long long w_cwait = 0, w_cwork = 0;
@@ -676,21 +648,21 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
       const __half2* szp  = reinterpret_cast<const __half2*>(pr->scale_b) + gn;
       // K blocks per (scale, zero) group as a shift: 1 for groups of 128 (two 64-k stages); the per-channel scheme
       // (cta_gemm.cuh:112-286) has one group for the whole of K
-      // (with stages of two K blocks a stage IS a group of 128)
-      const int gsh       = pr->one_group ? 30 : (kTwo ? 0 : 1);
+      const int gsh       = pr->one_group ? 30 : 1;
       const int kb_first  = (int)(((uint32_t)group + kCvtGroups - it % kCvtGroups) % kCvtGroups);   // first K block of this tile the group handles
       __half2 sz_next = __float2half2_rn(0.f);
       if (has_sz && kb_first < ti.nkb) sz_next = __ldg(szp + (int64_t)(kb_first >> gsh) * N);
       for (int kb = 0; kb < ti.nkb; ++kb, ++it) {
-        const int s_cur       = stage;
-        const uint32_t ph_cur = phase;
-        if (++stage == G::kStages) { stage = 0; phase ^= 1u; }
+        const int s_cur       = stage, wb_cur = wb;
+        const uint32_t ph_cur = wphase;
+        if (++stage == G::kStages) stage = 0;
+        if (++wb == G::kWBars) { wb = 0; wphase ^= 1u; }
         if ((int)(it % kCvtGroups) != group) continue;   // another group's stage
         const __half2 sz = sz_next;
         if (has_sz && kb + kCvtGroups < ti.nkb) sz_next = __ldg(szp + (int64_t)((kb + kCvtGroups) >> gsh) * N);
         const long long c0 = tick(prof_on);
         if (!dead) {
-          const bool ok = warp_wait_bar(smem_u32(&ctrl->wfull[s_cur]), ph_cur, abort_flag, lane, tmo);
+          const bool ok = warp_wait_bar(smem_u32(&ctrl->wfull[wb_cur]), ph_cur, abort_flag, lane, tmo);
           if (!ok) {
             if (lane == 0) report_s(status, convert ? 5 : 6, t);
             dead = true;
@@ -705,17 +677,12 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
         if (q == 0 && lane == 0) TRACE(TR_CVT_GOT, (int)it);
         if (convert) {
           tc_fence_after_sync();
-          // stages of two K blocks: the second block's packed weights lie behind the first's, its converted form
-          // goes to the upper 32 columns of the stage's A slot
-          const int nb = (kTwo && !(ti.odd && kb + 1 == ti.nkb)) ? 2 : 1;
-#pragma unroll 1
-          for (int b = 0; b < nb; ++b) {
           uint32_t o[32];
           if (ti.scheme == SCH_W4A4_XA || ti.scheme == SCH_W4A4) {
             // packed row: 64 bytes, 16-byte chunks swizzled by (row >> 1) & 3 (64-byte swizzle of the tensor map).
             // Chunk c becomes 32 int8 bytes: its high nibbles, then its low nibbles, each moved to the top of a
             // byte (code q -> byte 16*q; the accumulator is shifted back in the epilogue).
-            const uint32_t src = wslot(s_cur) + b * (kWSlotBytes / 2) + row * 64;
+            const uint32_t src = wslot(s_cur) + row * 64;
             const int sw       = (row >> 1) & 3;
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
@@ -730,7 +697,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
             // stage is the 16-byte chunk 2*kb16 + (f >> 1) (128-byte swizzle: XOR r), nibble 2*(f & 1) + c of
             // word d holds k = 16*kb16 + 8*c + d.
             const int f = lane >> 3, r = lane & 7;
-            const uint32_t src = wslot(s_cur) + b * (kWSlotBytes / 4) + (8 * q + r) * 128;
+            const uint32_t src = wslot(s_cur) + (8 * q + r) * 128;
             const __half2 s2 = __half2half2(__low2half(sz)), z2 = __half2half2(__high2half(sz));
 #pragma unroll
             for (int kb16 = 0; kb16 < 4; ++kb16) {
@@ -745,8 +712,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
               }
             }
           }
-          tmem_st_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + G::kASlotCol0 + s_cur * G::kASlotStride + b * kASlotCols, o);
-          }
+          tmem_st_32x32(tmem_base + ((uint32_t)(q * 32) << 16) + G::kASlotCol0 + s_cur * kASlotCols, o);
           if (kMode == 2 && ti.scheme == SCH_W4A4) {
             // packed activation rows -> int8 rows of the swizzled operand tile (the same nibble -> byte 16*q map)
             const int rows32 = (ti.ntok + 31) & ~31;
@@ -757,6 +723,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
         // the stage's packed weights are in registers (or not needed): release the stage
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&ctrl->empty[s_cur]));
+        __syncwarp();   // (tcgen05.wait and bar.arrive take the whole warp)
         if (convert) {
           tmem_st_wait();
           tc_fence_before_sync();
@@ -790,18 +757,16 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
 }
 
 namespace {
-template <int kMode, bool kSmall>
+template <int kMode>
 cudaError_t configure_one() {
-  cudaError_t e = cudaFuncSetAttribute(gg_swap_kernel<kMode, kSmall, false>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes_swap<Geo<kSmall>>());
+  cudaError_t e = cudaFuncSetAttribute(gg_swap_kernel<kMode, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(gg_swap_kernel<kMode, kSmall, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              smem_bytes_swap<Geo<kSmall>>());
+  return cudaFuncSetAttribute(gg_swap_kernel<kMode, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
 }
-template <int kMode, bool kSmall>
+template <int kMode>
 void launch_one(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
-  if (ext) gg_swap_kernel<kMode, kSmall, true><<<num_ctas, CfgS<kMode>::kThreads, smem_bytes_swap<Geo<kSmall>>(), stream>>>(problems, count, status);
-  else     gg_swap_kernel<kMode, kSmall, false><<<num_ctas, CfgS<kMode>::kThreads, smem_bytes_swap<Geo<kSmall>>(), stream>>>(problems, count, status);
+  if (ext) gg_swap_kernel<kMode, true><<<num_ctas, CfgS<kMode>::kThreads, kSmemBytes, stream>>>(problems, count, status);
+  else     gg_swap_kernel<kMode, false><<<num_ctas, CfgS<kMode>::kThreads, kSmemBytes, stream>>>(problems, count, status);
 }
 }  // namespace
 
@@ -813,26 +778,16 @@ extern "C" int mxmoe_gg_trace(long long* out) {   // out[kTraceEvents][kTraceLen
 
 cudaError_t gg_configure_swap() {
   cudaError_t e;
-  if ((e = configure_one<0, false>()) != cudaSuccess) return e;
-  if ((e = configure_one<1, false>()) != cudaSuccess) return e;
-  if ((e = configure_one<2, false>()) != cudaSuccess) return e;
-  if ((e = configure_one<0, true>()) != cudaSuccess) return e;
-  if ((e = configure_one<1, true>()) != cudaSuccess) return e;
-  if ((e = configure_one<2, true>()) != cudaSuccess) return e;
-  return cudaSuccess;
+  if ((e = configure_one<0>()) != cudaSuccess) return e;
+  if ((e = configure_one<1>()) != cudaSuccess) return e;
+  return configure_one<2>();
 }
 
-void gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool small_tiles,
-                    bool ext, int num_ctas, cudaStream_t stream) {
-  if (small_tiles) {
-    if (cvt_mode == 2)  launch_one<2, true>(problems, count, status, ext, num_ctas, stream);
-    else if (cvt_mode)  launch_one<1, true>(problems, count, status, ext, num_ctas, stream);
-    else                launch_one<0, true>(problems, count, status, ext, num_ctas, stream);
-  } else {
-    if (cvt_mode == 2)  launch_one<2, false>(problems, count, status, ext, num_ctas, stream);
-    else if (cvt_mode)  launch_one<1, false>(problems, count, status, ext, num_ctas, stream);
-    else                launch_one<0, false>(problems, count, status, ext, num_ctas, stream);
-  }
+void gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
+                    cudaStream_t stream) {
+  if (cvt_mode == 2)  launch_one<2>(problems, count, status, ext, num_ctas, stream);
+  else if (cvt_mode)  launch_one<1>(problems, count, status, ext, num_ctas, stream);
+  else                launch_one<0>(problems, count, status, ext, num_ctas, stream);
 }
 
 }  // namespace mxb

@@ -25,7 +25,6 @@ constexpr int kMaxRecs = 512;   // tiles per CTA kept in the table; later ones a
 
 struct TileS {
   int p, scheme, nkb, x_row, n_tile, ntok, c_row;
-  int odd;   // stages of two K blocks: the last stage holds one
 };
 
 __device__ __forceinline__ void report_s(GGStatus* status, int role, int tile) {
@@ -51,7 +50,7 @@ __device__ __forceinline__ TileRec make_rec(const Sched* sc, int count, int t, i
   if (pair_rank >= 0) ti.n_tile = 2 * ti.n_tile + pair_rank;
   const int tile_tok = ti.scheme == SCH_W4A4 ? tok_packed : tok;   // problems with packed activations: shorter tiles
   TileRec r;
-  r.pk     = ti.p | (ti.scheme << 8) | (ti.nkb << 12) | (ti.odd << 30);
+  r.pk     = ti.p | (ti.scheme << 8) | (ti.nkb << 12);
   r.x_row  = sc->row0[ti.p] + ti.m_tile * tile_tok;
   r.nt     = ti.n_tile | (min(tile_tok, sc->m_eff[ti.p] - ti.m_tile * tile_tok) << 16);
   r.c_row  = r.x_row + sc->c_shift[ti.p];
@@ -72,7 +71,7 @@ __device__ __forceinline__ void acquire_tile_maps(const GGSwapProblemDev* proble
 }
 __device__ __forceinline__ TileS decode_rec(const TileRec& r) {
   TileS t;
-  t.p = r.pk & 0xff; t.scheme = (r.pk >> 8) & 15; t.nkb = (r.pk >> 12) & 0x3FFFF; t.odd = (r.pk >> 30) & 1;
+  t.p = r.pk & 0xff; t.scheme = (r.pk >> 8) & 15; t.nkb = (r.pk >> 12) & 0x3FFFF;
   t.x_row = r.x_row; t.n_tile = r.nt & 0xffff; t.ntok = r.nt >> 16; t.c_row = r.c_row;
   return t;
 }
@@ -115,7 +114,6 @@ __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
 // TMEM lane quarter, so every instruction it does not need (a predicate set-up per MMA, descriptor arithmetic
 // recomputed per stage) delays the issue of the next stage.  `first` == 0: the first MMA overwrites D.
 //   kV 0 int8 / weights from shared memory, 1 fp16 / shared memory, 2 int8 / tensor memory, 3 fp16 / tensor memory.
-#define MXB_COMMIT1 "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"
 #define MXB_MMA_STAGE_SS(KIND)                                                                              \
   asm volatile(                                                                                             \
       "{\n\t"                                                                                               \
@@ -137,7 +135,7 @@ __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
       :                                                                                                     \
       : "r"(d_tmem), "r"(wlo), "r"(xlo), "r"(desc_hi), "r"(idesc), "r"(first), "r"(empty_bar)               \
       : "memory")
-#define MXB_MMA_STAGE_TS(KIND, COMMIT)                                                                      \
+#define MXB_MMA_STAGE_TS(KIND)                                                                              \
   asm volatile(                                                                                             \
       "{\n\t"                                                                                               \
       ".reg .pred p, t;\n\t"                                                                                \
@@ -152,7 +150,7 @@ __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
       "tcgen05.mma.cta_group::1.kind::" KIND " [%0], [a1], x1, %4, t;\n\t"                                  \
       "tcgen05.mma.cta_group::1.kind::" KIND " [%0], [a2], x2, %4, t;\n\t"                                  \
       "tcgen05.mma.cta_group::1.kind::" KIND " [%0], [a3], x3, %4, t;\n\t"                                  \
-      COMMIT                                                                                                \
+      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%6];\n\t"                     \
       "}"                                                                                                   \
       :                                                                                                     \
       : "r"(d_tmem), "r"(a_tmem), "r"(xlo), "r"(desc_hi), "r"(idesc), "r"(first), "r"(empty_bar)            \
@@ -204,8 +202,7 @@ __device__ __forceinline__ void sts32(uint32_t addr, uint32_t v) {
         "h"((unsigned short)3)                                                                              \
       : "memory")
 
-// kCommit = false (weights from tensor memory, single CTAs): the first K block of a stage that holds two
-template <int kV, bool kPair, bool kCommit = true>
+template <int kV, bool kPair>
 __device__ __forceinline__ void mma_stage(uint32_t d_tmem, uint32_t wlo, uint32_t a_tmem, uint32_t xlo, uint32_t desc_hi,
                                           uint32_t idesc, uint32_t first, uint32_t empty_bar) {
   if (kPair) {
@@ -216,8 +213,8 @@ __device__ __forceinline__ void mma_stage(uint32_t d_tmem, uint32_t wlo, uint32_
   } else {
     if (kV == 0)      { MXB_MMA_STAGE_SS("i8"); }
     else if (kV == 1) { MXB_MMA_STAGE_SS("f16"); }
-    else if (kV == 2) { if (kCommit) { MXB_MMA_STAGE_TS("i8", MXB_COMMIT1); } else { MXB_MMA_STAGE_TS("i8", ""); } }
-    else              { if (kCommit) { MXB_MMA_STAGE_TS("f16", MXB_COMMIT1); } else { MXB_MMA_STAGE_TS("f16", ""); } }
+    else if (kV == 2) { MXB_MMA_STAGE_TS("i8"); }
+    else              { MXB_MMA_STAGE_TS("f16"); }
   }
 }
 

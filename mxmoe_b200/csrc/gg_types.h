@@ -56,7 +56,7 @@ static_assert(sizeof(GGProblemDev) == 384, "GGProblemDev layout");
 constexpr int kWT = 128;   // output channels per tile (tcgen05 M)
 constexpr int kTT = 176;   // tokens per tile (tcgen05 N, any multiple of 16 up to this)
 // the kernel on CTA pairs (gg_duo_kernel.cu): tokens per tile without / with 4-bit weights in the launch
-constexpr int kDuoTok = 256, kDuoTokCvt = 192;
+constexpr int kDuoTok = 256, kDuoTokCvt = 192, kDuoTokShort = 32;   // (short: launches with few rows per problem)
 constexpr int kXBoxSmall = 32;   // rows of the small activation box (short token tiles load only what they need)
 struct alignas(128) GGSwapProblemDev {
   CUtensorMap tmW;    // weights: 128 channels x one stage of K (packed for the 4-bit schemes)
@@ -124,15 +124,14 @@ cudaError_t gg_launch_pair(const GGProblemDev* problems, int count, GGStatus* st
                            cudaStream_t stream);
 cudaError_t gg_configure_pair();
 // kernel with swapped operands (gg_swap_kernel.cu): weights from tensor memory / shared memory as the M side,
-// token tiles of up to 176 rows (ring of 5 stages) or, with `small_tiles`, of up to 32 rows (ring of 10 stages)
-// as the N side
+// token tiles of up to 176 rows as the N side
 // `ext`: the launch holds problems with an optional result form (weight maps of rank 4), see gg_swap_kernel
-void gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool small_tiles, bool ext,
-                    int num_ctas, cudaStream_t stream);
+void gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
+                    cudaStream_t stream);
 cudaError_t gg_configure_swap();
-// CTA pairs (gg_duo_kernel.cu); num_ctas >= 2
-void gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
-                   cudaStream_t stream);
+// CTA pairs (gg_duo_kernel.cu); num_ctas >= 2; `short_tiles`: token tiles of 32 rows
+void gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool short_tiles, bool ext,
+                   int num_ctas, cudaStream_t stream);
 cudaError_t gg_configure_duo();
 
 }  // namespace mxb

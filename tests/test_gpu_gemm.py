@@ -19,14 +19,15 @@ pytestmark = pytest.mark.gpu
 REL_L2 = 1e-3
 
 
-@pytest.fixture(autouse=True, params=["swap", "swap-small", "swap2", "pair", "single"])
+@pytest.fixture(autouse=True, params=["swap", "swap-small", "swap2", "swap2-small", "pair", "single"])
 def gg_kernel(request, monkeypatch):
     """Every test of this file runs once per kernel: swapped operands (128 channels x up to 176 tokens, 4-bit
-    weights through tensor memory; "swap-small" forces its geometry for few rows - 32-token tiles, ring of 10 stages -
-    on every shape), CTA pairs (256 x 256 tiles, cta_group::2) and single CTAs (128 x 256 tiles)."""
+    weights through tensor memory), the same on CTA pairs (256 channels x up to 256 tokens; "swap2-small" forces its
+    geometry for few rows - 32-token tiles, ring of 10 stages - on every shape), CTA pairs with tokens as the M side
+    (256 x 256 tiles, cta_group::2) and single CTAs (128 x 256 tiles)."""
     kernel = request.param.split("-")[0]
     monkeypatch.setenv("MXMOE_GG_KERNEL", kernel)
-    if request.param == "swap-small":
+    if request.param.endswith("-small"):
         monkeypatch.setenv("MXMOE_GG_TILES", "small")
     else:
         monkeypatch.delenv("MXMOE_GG_TILES", raising=False)
