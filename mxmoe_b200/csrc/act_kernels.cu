@@ -27,6 +27,7 @@
 #include <cstdint>
 
 #include "act_kernels.h"
+#include "launch.cuh"
 
 namespace mxb {
 namespace {
@@ -380,6 +381,8 @@ __device__ __forceinline__ void emit_row_multi(const float (&x)[kJ][8], float am
 // fused gather + (rotate) + quantise, one pass per routed row (operator-API path, any top-k)
 template <int kWarps>
 __global__ void __launch_bounds__(kBlock) quant_act_kernel(ActArgs a) {
+  release_dependents();
+  grid_dependency_wait();
   __shared__ float xch[kWarps > 1 ? kBlock * 8 : 1];
   __shared__ float red[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -418,6 +421,8 @@ __global__ void __launch_bounds__(kBlock) quant_act_kernel(ActArgs a) {
 // (rotate) + quantise once per token into token-major stores, one per activation format in use
 template <int kWarps>
 __global__ void __launch_bounds__(kBlock, 3) quant_tokens_kernel(TokenQuantArgs a) {
+  release_dependents();
+  grid_dependency_wait();
   __shared__ float xch[kWarps > 1 ? kBlock * 8 : 1];
   __shared__ float red[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -452,6 +457,8 @@ __global__ void __launch_bounds__(kBlock, 3) quant_tokens_kernel(TokenQuantArgs 
 template <int kWarps>
 __global__ void __launch_bounds__(kBlock, 2) quant_tokens_scatter_kernel(TokenQuantArgs a, ActArgs r, const int* slot_row,
                                                                          int topk) {
+  release_dependents();
+  grid_dependency_wait();
   __shared__ float xch[kWarps > 1 ? kBlock * 8 : 1];
   __shared__ float red[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -502,6 +509,8 @@ __global__ void __launch_bounds__(kBlock, 2) quant_tokens_scatter_kernel(TokenQu
 // copy every routed (and shared-expert) row from the token-major store of its expert's format into
 // the expert-sorted activation store; one warp per row, 16-byte chunks
 __global__ void __launch_bounds__(kBlock) gather_rows_kernel(ActArgs a, TokenQuantArgs t) {
+  release_dependents();
+  grid_dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = blockIdx.x * 8 + warp;
   if (row >= a.rows_total) return;
@@ -523,6 +532,8 @@ __global__ void __launch_bounds__(kBlock) gather_rows_kernel(ActArgs a, TokenQua
 // only the quantiser runs, on the same registers.
 template <int kWarps, bool kSilu>
 __device__ __forceinline__ void rows_quant_body(const ActArgs& a) {
+  release_dependents();
+  grid_dependency_wait();
   __shared__ float red[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row_in_blk = warp / kWarps, w = warp % kWarps;
@@ -629,13 +640,11 @@ __global__ void __launch_bounds__(kBlock, 3) silu_mul_quant_kernel(ActArgs a) { 
 template <int kWarps>
 __global__ void __launch_bounds__(kBlock, 3) rows_quant_kernel(ActArgs a) { rows_quant_body<kWarps, false>(a); }
 
-#define MXB_DISPATCH_WARPS(kmax, rows, KERNEL, ...)                                                   \
-  do {                                                                                                \
-    if ((kmax) <= 2048)      KERNEL<1><<<((rows) + 7) / 8, kBlock, 0, stream>>>(__VA_ARGS__);          \
-    else if ((kmax) <= 4096) KERNEL<2><<<((rows) + 3) / 4, kBlock, 0, stream>>>(__VA_ARGS__);          \
-    else if ((kmax) <= 8192) KERNEL<4><<<((rows) + 1) / 2, kBlock, 0, stream>>>(__VA_ARGS__);          \
-    else                     KERNEL<8><<<(rows), kBlock, 0, stream>>>(__VA_ARGS__);                    \
-  } while (0)
+#define MXB_DISPATCH_WARPS(kmax, rows, KERNEL, ...)                                                              \
+  ((kmax) <= 2048   ? launch_dependent(KERNEL<1>, ((rows) + 7) / 8, kBlock, 0, stream, __VA_ARGS__)              \
+   : (kmax) <= 4096 ? launch_dependent(KERNEL<2>, ((rows) + 3) / 4, kBlock, 0, stream, __VA_ARGS__)              \
+   : (kmax) <= 8192 ? launch_dependent(KERNEL<4>, ((rows) + 1) / 2, kBlock, 0, stream, __VA_ARGS__)              \
+                    : launch_dependent(KERNEL<8>, (rows), kBlock, 0, stream, __VA_ARGS__))
 
 }  // namespace
 
@@ -644,38 +653,32 @@ cudaError_t launch_quant_act(const ActArgs& a, cudaStream_t stream) {
   const int kmax = a.k > a.k_shared ? a.k : a.k_shared;
   if (!a.rotate && !a.row_token) {
     // rows in place, no rotation: the quantiser alone (the second half of silu_mul_quant)
-    MXB_DISPATCH_WARPS(kmax, a.rows_total, rows_quant_kernel, a);
-  } else {
-    MXB_DISPATCH_WARPS(kmax, a.rows_total, quant_act_kernel, a);
+    return MXB_DISPATCH_WARPS(kmax, a.rows_total, rows_quant_kernel, a);
   }
-  return cudaGetLastError();
+  return MXB_DISPATCH_WARPS(kmax, a.rows_total, quant_act_kernel, a);
 }
 
 cudaError_t launch_silu_mul_quant(const ActArgs& a, cudaStream_t stream) {
   if (a.rows_total <= 0) return cudaSuccess;
   const int kmax = a.k > a.k_shared ? a.k : a.k_shared;
-  MXB_DISPATCH_WARPS(kmax, a.rows_total, silu_mul_quant_kernel, a);
-  return cudaGetLastError();
+  return MXB_DISPATCH_WARPS(kmax, a.rows_total, silu_mul_quant_kernel, a);
 }
 
 cudaError_t launch_quant_tokens(const TokenQuantArgs& t, cudaStream_t stream) {
   if (t.num_tokens <= 0) return cudaSuccess;
-  MXB_DISPATCH_WARPS(t.k, t.num_tokens, quant_tokens_kernel, t);
-  return cudaGetLastError();
+  return MXB_DISPATCH_WARPS(t.k, t.num_tokens, quant_tokens_kernel, t);
 }
 
 cudaError_t launch_quant_tokens_scatter(const TokenQuantArgs& t, const ActArgs& r, const int* slot_row, int topk,
                                         cudaStream_t stream) {
   if (t.num_tokens <= 0) return cudaSuccess;
   if (topk < 1 || topk > kMaxDst) return cudaErrorInvalidValue;
-  MXB_DISPATCH_WARPS(t.k, t.num_tokens, quant_tokens_scatter_kernel, t, r, slot_row, topk);
-  return cudaGetLastError();
+  return MXB_DISPATCH_WARPS(t.k, t.num_tokens, quant_tokens_scatter_kernel, t, r, slot_row, topk);
 }
 
 cudaError_t launch_gather_rows(const ActArgs& a, const TokenQuantArgs& t, cudaStream_t stream) {
   if (a.rows_total <= 0) return cudaSuccess;
-  gather_rows_kernel<<<(a.rows_total + 7) / 8, kBlock, 0, stream>>>(a, t);
-  return cudaGetLastError();
+  return launch_dependent(gather_rows_kernel, (a.rows_total + 7) / 8, kBlock, 0, stream, a, t);
 }
 
 }  // namespace mxb

@@ -36,6 +36,7 @@
 // have landed.  Every wait is bounded; a role whose wait runs out reports, raises the
 // CTA's abort flag and leaves its loop, the others follow by the flag or by their own limit.
 #include "gg_tile.cuh"
+#include "launch.cuh"
 
 namespace mxb {
 
@@ -181,6 +182,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
   if (count > kMaxProblems) {
+    grid_dependency_wait();
     if (tid == 0 && blockIdx.x == 0) atomicCAS(&status->error, 0, kDevErrTooMany);
     return;
   }
@@ -202,6 +204,11 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
     ctrl->timeout_ns = status->timeout_ms > 0 ? (uint64_t)status->timeout_ms * 1000000ull : kTimeoutNs;
     fence_mbar_init();
   }
+  if (warp == 1) {
+    tmem_alloc2(smem_u32(&ctrl->tmem_base), 512);
+    tmem_relinquish2();
+  }
+  grid_dependency_wait();   // row counts and operands come from the kernels before this one
   build_sched(sc, problems, count, G::kTok, 2 * kWT, G::kTok);
   const int total_tiles = sc->total_tiles;
   const int my_tiles    = total_tiles > cta ? (total_tiles - cta + nctas - 1) / nctas : 0;
@@ -212,10 +219,6 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
     if (i < kDuoRecs) return ctrl->recs[i];
     return make_rec(sc, count, cta + i * nctas, G::kTok, G::kTok, rank);
   };
-  if (warp == 1) {
-    tmem_alloc2(smem_u32(&ctrl->tmem_base), 512);
-    tmem_relinquish2();
-  }
   tc_fence_before_sync();
   __syncthreads();
   cluster_sync_all();   // both CTAs' barriers exist before either signals the other's
@@ -699,8 +702,8 @@ cudaError_t configure_duo() {
 template <int kMode, bool kShort>
 void launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
   using G = DuoGeo<kMode, kShort>;
-  if (ext) gg_duo_kernel<kMode, kShort, true><<<num_ctas & ~1, G::kThreads, smem_bytes_duo<G>(), stream>>>(problems, count, status);
-  else     gg_duo_kernel<kMode, kShort, false><<<num_ctas & ~1, G::kThreads, smem_bytes_duo<G>(), stream>>>(problems, count, status);
+  launch_dependent(ext ? gg_duo_kernel<kMode, kShort, true> : gg_duo_kernel<kMode, kShort, false>, num_ctas & ~1, G::kThreads,
+                   smem_bytes_duo<G>(), stream, problems, count, status);
 }
 template <bool kShort>
 void launch_mode(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas, cudaStream_t stream) {

@@ -50,6 +50,7 @@
 // walking its loop without waiting or working, so that every bar.arrive another warp counts on is still made
 // and the kernel ends.
 #include "gg_tile.cuh"
+#include "launch.cuh"
 
 namespace mxb {
 
@@ -193,6 +194,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
   const int lane = tid & 31;
 
   if (count > kMaxProblems) {
+    grid_dependency_wait();
     if (tid == 0 && blockIdx.x == 0) atomicCAS(&status->error, 0, kDevErrTooMany);
     return;
   }
@@ -215,6 +217,11 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
     ctrl->abort_flag = 0;
     fence_mbar_init();
   }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&ctrl->tmem_base), 512);
+    tmem_relinquish();
+  }
+  grid_dependency_wait();   // row counts and operands come from the kernels before this one
   // problems with packed 4-bit activations use token tiles of at most 128 rows: the packed rows of a stage
   // (128 x 64 B) then fit behind the packed weights in the stage's weight slot
   constexpr int kTokPacked = 128;
@@ -228,10 +235,6 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
     if (i < kMaxRecs) return ctrl->recs[i];
     return make_rec(sc, count, cta + i * nctas, G::kTok, kTokPacked);
   };
-  if (warp == 1) {
-    tmem_alloc(smem_u32(&ctrl->tmem_base), 512);
-    tmem_relinquish();
-  }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
@@ -765,8 +768,8 @@ cudaError_t configure_one() {
 }
 template <int kMode>
 void launch_one(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
-  if (ext) gg_swap_kernel<kMode, true><<<num_ctas, CfgS<kMode>::kThreads, kSmemBytes, stream>>>(problems, count, status);
-  else     gg_swap_kernel<kMode, false><<<num_ctas, CfgS<kMode>::kThreads, kSmemBytes, stream>>>(problems, count, status);
+  launch_dependent(ext ? gg_swap_kernel<kMode, true> : gg_swap_kernel<kMode, false>, num_ctas, CfgS<kMode>::kThreads, kSmemBytes,
+                   stream, problems, count, status);
 }
 }  // namespace
 

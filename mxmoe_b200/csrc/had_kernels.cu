@@ -14,6 +14,7 @@
 // hot loops: at 8192 tokens x top-4 it is 16 GFLOP beside the layer's 567 GFLOP, and it is bounded by reading and
 // writing the rows once (2 x 92 MB).
 #include "had_kernels.h"
+#include "launch.cuh"
 
 #include <cstdint>
 
@@ -39,6 +40,8 @@ template <int KP, bool kFwht8>
 __global__ void __launch_bounds__(kThreads) had_kron_kernel(const __half* __restrict__ in, __half* __restrict__ out,
                                                             const __half* __restrict__ hadK, int rows, int K, int m,
                                                             float scale) {
+  release_dependents();
+  grid_dependency_wait();
   constexpr int LD = KP + 8;                         // row pitch of both shared tiles (halfs): keeps ldmatrix conflict-free
   extern __shared__ __align__(16) uint8_t smem[];
   __half* sH = reinterpret_cast<__half*>(smem);      // [KP][LD]   hadK[a][a']
@@ -167,9 +170,7 @@ cudaError_t launch(const __half* in, __half* out, const __half* hadK, int rows, 
   const long long tiles = (long long)((rows + kRowsPerBlock - 1) / kRowsPerBlock) * (m >> 3);
   const int per_sm = smem > 100 * 1024 ? 2 : 4;
   const int grid = (int)(tiles < (long long)sms * per_sm ? tiles : (long long)sms * per_sm);
-  if (fwht8) k1<<<grid, kThreads, smem, stream>>>(in, out, hadK, rows, K, m, scale);
-  else       k0<<<grid, kThreads, smem, stream>>>(in, out, hadK, rows, K, m, scale);
-  return cudaGetLastError();
+  return launch_dependent(fwht8 ? k1 : k0, grid, kThreads, smem, stream, in, out, hadK, rows, K, m, scale);
 }
 
 }  // namespace

@@ -9,6 +9,7 @@
 // directly.  Rows of one expert keep the order of the flattened (token, slot)
 // index, i.e. the result equals a stable sort.
 #include "route_kernels.h"
+#include "launch.cuh"
 
 #include <cuda_fp16.h>
 
@@ -33,6 +34,8 @@ __device__ __forceinline__ int read_id(const RouteArgs& a, int idx) {
 }
 
 __global__ void __launch_bounds__(kThreads) route_count_kernel(RouteArgs a) {
+  release_dependents();
+  grid_dependency_wait();
   __shared__ int hist[kMaxE];
   const int n = a.num_tokens * a.topk;
   for (int e = threadIdx.x; e < a.num_experts; e += kThreads) hist[e] = 0;
@@ -54,6 +57,8 @@ __global__ void __launch_bounds__(kThreads) route_count_kernel(RouteArgs a) {
 // the blocks with a load -> store chain per step cost a global-memory latency per block.
 constexpr int kScanThreads = 1024;
 __global__ void __launch_bounds__(kScanThreads) route_scan_kernel(RouteArgs a, int nblocks) {
+  release_dependents();
+  grid_dependency_wait();
   __shared__ int total[kMaxE];
   __shared__ int start[kMaxE + 1];
   const int E = a.num_experts;
@@ -103,6 +108,8 @@ __global__ void __launch_bounds__(kScanThreads) route_scan_kernel(RouteArgs a, i
 // the row offsets itself, so the count and scan launches are not needed and no workspace is read.
 template <bool kSingle>
 __global__ void __launch_bounds__(kThreads) route_scatter_kernel(RouteArgs a) {
+  release_dependents();
+  grid_dependency_wait();
   __shared__ int wbase[kThreads / 32][kMaxE];
   __shared__ int start[kSingle ? kMaxE + 1 : 1];
   const int n    = a.num_tokens * a.topk;
@@ -181,6 +188,8 @@ __global__ void __launch_bounds__(kThreads) route_scatter_kernel(RouteArgs a) {
 __global__ void __launch_bounds__(kThreads) combine_kernel(const __half* __restrict__ y, const int* __restrict__ slot_row,
                                                            const float* __restrict__ w, const __half* __restrict__ ysh,
                                                            __half* __restrict__ out, int topk, int hidden) {
+  release_dependents();
+  grid_dependency_wait();
   const int t = blockIdx.x;
   for (int c = threadIdx.x; c < hidden / 8; c += kThreads) {
     float acc[8];
@@ -223,6 +232,8 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const __half* __restr
 template <typename T>
 __global__ void __launch_bounds__(kThreads) gate_topk_kernel(const T* __restrict__ logits, int num_tokens, int E, int topk,
                                                              int renorm, int* __restrict__ ids, float* __restrict__ wts) {
+  release_dependents();
+  grid_dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int t = blockIdx.x * (kThreads / 32) + warp;
   if (t >= num_tokens) return;
@@ -284,9 +295,9 @@ cudaError_t launch_gate_topk(const void* logits, bool fp16, int num_tokens, int 
   if (num_tokens <= 0) return cudaSuccess;
   if (num_experts > kMaxE || topk > 32 || topk > num_experts) return cudaErrorInvalidValue;
   const int blocks = (num_tokens + kThreads / 32 - 1) / (kThreads / 32);
-  if (fp16) gate_topk_kernel<__half><<<blocks, kThreads, 0, stream>>>(static_cast<const __half*>(logits), num_tokens, num_experts, topk, renorm, ids, wts);
-  else      gate_topk_kernel<float><<<blocks, kThreads, 0, stream>>>(static_cast<const float*>(logits), num_tokens, num_experts, topk, renorm, ids, wts);
-  return cudaGetLastError();
+  if (fp16)
+    return launch_dependent(gate_topk_kernel<__half>, blocks, kThreads, 0, stream, static_cast<const __half*>(logits), num_tokens, num_experts, topk, renorm, ids, wts);
+  return launch_dependent(gate_topk_kernel<float>, blocks, kThreads, 0, stream, static_cast<const float*>(logits), num_tokens, num_experts, topk, renorm, ids, wts);
 }
 
 size_t route_workspace_bytes(int num_tokens, int topk, int num_experts) {
@@ -299,14 +310,13 @@ cudaError_t launch_route(const RouteArgs& a, cudaStream_t stream) {
   const int n = a.num_tokens * a.topk;
   const int nblocks = (n + kChunk - 1) / kChunk;
   if (a.num_experts > kMaxE) return cudaErrorInvalidValue;
-  if (nblocks == 1) {   // a decode batch: one launch does all three steps
-    route_scatter_kernel<true><<<1, kThreads, 0, stream>>>(a);
-    return cudaGetLastError();
-  }
-  if (nblocks > 0) route_count_kernel<<<nblocks, kThreads, 0, stream>>>(a);
-  route_scan_kernel<<<1, kScanThreads, 0, stream>>>(a, nblocks);
-  if (nblocks > 0) route_scatter_kernel<false><<<nblocks, kThreads, 0, stream>>>(a);
-  return cudaGetLastError();
+  if (nblocks == 1)   // a decode batch: one launch does all three steps
+    return launch_dependent(route_scatter_kernel<true>, 1, kThreads, 0, stream, a);
+  cudaError_t e;
+  if (nblocks > 0 && (e = launch_dependent(route_count_kernel, nblocks, kThreads, 0, stream, a)) != cudaSuccess) return e;
+  if ((e = launch_dependent(route_scan_kernel, 1, kScanThreads, 0, stream, a, nblocks)) != cudaSuccess) return e;
+  if (nblocks > 0) return launch_dependent(route_scatter_kernel<false>, nblocks, kThreads, 0, stream, a);
+  return cudaSuccess;
 }
 
 
@@ -348,10 +358,8 @@ cudaError_t route_static_scratch_ptr(int** out) {
 cudaError_t launch_combine(const void* y, const int* slot_row, const float* topk_w, const void* y_shared, void* out,
                            int num_tokens, int topk, int hidden, cudaStream_t stream) {
   if (num_tokens <= 0) return cudaSuccess;
-  combine_kernel<<<num_tokens, kThreads, 0, stream>>>(static_cast<const __half*>(y), slot_row, topk_w,
-                                                      static_cast<const __half*>(y_shared), static_cast<__half*>(out),
-                                                      topk, hidden);
-  return cudaGetLastError();
+  return launch_dependent(combine_kernel, num_tokens, kThreads, 0, stream, static_cast<const __half*>(y), slot_row, topk_w,
+                          static_cast<const __half*>(y_shared), static_cast<__half*>(out), topk, hidden);
 }
 
 }  // namespace mxb
