@@ -571,20 +571,20 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
     const int q     = warp & 3;
     const int group = (warp - kFirstCvt) / kCvtGroup;
     const int row   = q * 32 + lane;
-    int stage = 0, wbar = 0;
-    uint32_t wphase = 0;                   // parity of the next use of wfull[wbar]
-    uint32_t nc = 0;                       // converted K blocks walked so far
-    uint32_t it = 0;                       // stages walked so far
-    uint32_t i1 = 0, i2 = 0, i3 = 0, i4 = 0;   // values of `it` of the last four converted K blocks
+    // Where a tile starts: stage, barrier of its first converted K block with the parity of its next use, A slot, the group
+    // whose turn it is, stages walked so far.  A group steps from one of its own K blocks to the next: its chain of dependent
+    // instructions is what bounds launches with 4-bit weights, so nothing is walked or divided per block.
+    int stage0 = 0, wbar0 = 0, slot0 = 0, turn = 0;
+    uint32_t wphase0 = 0, it0 = 0;
+    uint32_t i1 = -64, i2 = -64, i3 = -64, i4 = -64;   // stage counts of the last four converted K blocks before the tile (none: long ago)
     bool ok = true;
     TileRec nrec = tile_rec(0);
     for (int i = 0; ok && i < my_tiles; ++i) {
       const TileS ti = decode_rec(nrec);
       if (i + 1 < my_tiles) nrec = tile_rec(i + 1);
       if (!is_cvt_scheme(ti.scheme)) {
-        stage += ti.nkb;
-        it += ti.nkb;
-        stage %= G::kStages;
+        stage0 = (stage0 + ti.nkb) % G::kStages;
+        it0 += ti.nkb;
         continue;
       }
       const GGSwapProblemDev* pr = problems + ti.p;
@@ -594,18 +594,13 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       const bool has_sz   = ti.scheme == SCH_W4A16G128 && gn < N;
       const __half2* szp  = reinterpret_cast<const __half2*>(pr->scale_b) + gn;
       const int gsh       = pr->one_group ? 30 : 1;
-      const int kb_first  = (int)((group + kCvtGroups - nc % kCvtGroups) % kCvtGroups);
+      const int kb_first  = group >= turn ? group - turn : group + kCvtGroups - turn;
       __half2 sz_next = __float2half2_rn(0.f);
       if (has_sz && kb_first < ti.nkb) sz_next = __ldg(szp + (int64_t)(kb_first >> gsh) * N);
-      for (int kb = 0; kb < ti.nkb; ++kb, ++nc, ++it) {
-        const int s             = stage;
-        const int wb            = wbar;
-        const uint32_t wpar     = wphase;
-        const uint32_t last     = i4;      // K block nc - 4, the previous content of the A slot
-        if (++wbar == G::kWBars) { wbar = 0; wphase ^= 1u; }
-        i4 = i3; i3 = i2; i2 = i1; i1 = it;
-        if (++stage == G::kStages) stage = 0;
-        if ((int)(nc % kCvtGroups) != group) continue;
+      int s = (stage0 + kb_first) % G::kStages, wb = wbar0 + kb_first, slot = (slot0 + kb_first) % G::kASlots;
+      uint32_t wpar = wphase0;
+      if (wb >= G::kWBars) { wb -= G::kWBars; wpar ^= 1u; }
+      for (int kb = kb_first; kb < ti.nkb; kb += kCvtGroups) {
         const __half2 sz = sz_next;
         if (has_sz && kb + kCvtGroups < ti.nkb) sz_next = __ldg(szp + (int64_t)((kb + kCvtGroups) >> gsh) * N);
         if (!wwait<G>(smem_base, wfull0 + 8 * wb, wpar)) {
@@ -615,7 +610,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         }
         // The row's 128 bytes of the A slot are formed and stored in two halves of 16 words (fewer registers), the first
         // while the slot may still be in use.
-        const uint32_t a_addr = tmem_base + ((uint32_t)(q * 32) << 16) + G::kACol0 + (nc % G::kASlots) * kASlotCols;
+        const uint32_t a_addr = tmem_base + ((uint32_t)(q * 32) << 16) + G::kACol0 + slot * kASlotCols;
 #pragma unroll
         for (int hf = 0; hf < 2; ++hf) {
           uint32_t o[16];
@@ -653,14 +648,18 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
               convert_w4a4<kCvtGroup * 32>(wslot(s) + kWSlotBytes / 2, xslot(s), (half_rows + 31) & ~31, q * 32 + lane);
               fence_proxy_async_smem();
             }
-            // The slot's previous content has been read: the MMAs of converted K block nc - 4 have completed.  If that
-            // was a whole ring ago they have (this stage was refilled after the MMAs a ring back), and its barrier may
+            // The slot's previous content has been read: the MMAs of the fourth converted K block back have completed.  If
+            // that was a whole ring ago they have (this stage was refilled after the MMAs a ring back), and its barrier may
             // have moved on.
-            if (G::kASlots < G::kStages && nc >= (uint32_t)G::kASlots && it - last < (uint32_t)G::kStages &&
-                !wwait<G>(smem_base, empty0 + 8 * (last % G::kStages), (last / G::kStages) & 1u)) {
-              if (lane == 0) report_s(status, 6, cta + i * nctas);
-              ok = false;
-              break;
+            if (G::kASlots < G::kStages) {
+              const uint32_t it   = it0 + kb;
+              const uint32_t last = kb >= 4 ? it - 4 : (kb == 0 ? i4 : (kb == 1 ? i3 : (kb == 2 ? i2 : i1)));
+              if (it - last < (uint32_t)G::kStages &&
+                  !wwait<G>(smem_base, empty0 + 8 * (last % G::kStages), (last / G::kStages) & 1u)) {
+                if (lane == 0) report_s(status, 6, cta + i * nctas);
+                ok = false;
+                break;
+              }
             }
             tc_fence_after_sync();
           }
@@ -671,7 +670,21 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         tc_fence_before_sync();
         __syncwarp();
         if (lane == 0) mbar_arrive_leader_relaxed(full0 + 8 * s);
+        s += kCvtGroups;
+        if (s >= G::kStages) s -= G::kStages;
+        wb += kCvtGroups;
+        if (wb >= G::kWBars) { wb -= G::kWBars; wpar ^= 1u; }
+        slot += kCvtGroups;
+        if (slot >= G::kASlots) slot -= G::kASlots;
       }
+      for (int kb = max(ti.nkb - 4, 0); kb < ti.nkb; ++kb) { i4 = i3; i3 = i2; i2 = i1; i1 = it0 + kb; }
+      stage0  = (stage0 + ti.nkb) % G::kStages;
+      slot0   = (slot0 + ti.nkb) % G::kASlots;
+      turn    = (turn + ti.nkb) % kCvtGroups;
+      wbar0 += ti.nkb;
+      wphase0 ^= (uint32_t)(wbar0 / G::kWBars) & 1u;
+      wbar0 %= G::kWBars;
+      it0 += ti.nkb;
     }
   }
 
