@@ -143,8 +143,8 @@ enum mxmoe_gg_kernel {
   MXMOE_GG_KERNEL_SWAP = 3,   /* swapped operands: 128 channels x up to 176 tokens per tile (128 when a problem has
                                  packed 4-bit activations), 4-bit weights converted into tensor memory */
   MXMOE_GG_KERNEL_SWAP2 = 4   /* the default: the same on CTA pairs (tcgen05 cta_group::2), 256 channels x up to 256 tokens
-                                 (192 when a problem has 4-bit weights), each CTA loads half of the token tile; launches
-                                 with 32-token tiles or of a single CTA run SWAP */
+                                 (192 when a problem has 4-bit weights, 32 when every problem has few rows), each CTA loads
+                                 half of the token tile; launches of a single CTA run SWAP */
 };
 int mxmoe_gg_run_kernel(void* workspace, const mxmoe_gg_plan* plan, int kernel, int num_ctas, void* stream);
 

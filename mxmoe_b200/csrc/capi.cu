@@ -309,7 +309,7 @@ int default_kernel() {
   return GGK_SWAP2;
 }
 
-// token-tile geometry of the SWAP kernel: chosen from the row counts unless MXMOE_GG_TILES = small | large overrides
+// token-tile geometry of the CTA-pair kernel: chosen from the row counts unless MXMOE_GG_TILES = small | large overrides
 // it (read when a workspace is prepared)
 bool small_tiles_at_prepare(bool few_rows) {
   const char* e = getenv("MXMOE_GG_TILES");

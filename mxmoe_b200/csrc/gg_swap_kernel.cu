@@ -34,7 +34,7 @@
 //               operator API's input format; token tiles are then 128 rows) the group also expands the
 //               stage's packed activation rows into the swizzled int8 operand tile in shared memory.
 //
-// Barrier protocol (mbarriers).  wfull[s] "the weights of stage s (and packed activations, which the converters
+// Barrier protocol (mbarriers; the weights have one per stage of two turns of the ring, see Geo::kWBars).  wfull[s] "the weights of stage s (and packed activations, which the converters
 // expand) have landed"; xfull[s] "the activation tile of stage s has landed"; empty[s] "stage s may be refilled"
 // = the MMAs of the stage have completed (tcgen05.commit) and the stage's converter group has read its packed
 // operands.  Every barrier completes once per use of its stage, whatever the tile's scheme, so parities follow
