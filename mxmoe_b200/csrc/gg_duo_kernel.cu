@@ -13,7 +13,7 @@
 // pipe is the limit for 8- and 16-bit operands: 516-529 cycles per stage of 512.  The chip then runs at its power
 // limit (1000 W at 1.2-1.3 GHz): fp16 1215 and int8 2413 TFLOP/s held for seconds, cuBLAS on the same operands 1211 and
 // 2322.  8 x [4096, 2816, 2048], short runs, us, single CTAs -> pairs: w8a8 172 -> 132, fp16 325 -> 270, w4a4 162 -> 143
-// (packed activations 310 -> 186), w4a16 389 -> 334; 8 x [4096, 2048, 1408]: 109 -> 75, 172 -> 140, 124 -> 88 (184 -> 109),
+// (packed activations 310 -> 243), w4a16 389 -> 334; 8 x [4096, 2048, 1408]: 109 -> 75, 172 -> 140, 124 -> 88 (184 -> 137),
 // 213 -> 175.
 //
 // Tiles.  Without 4-bit weights 256 tokens (both accumulators fill tensor memory), ring of six 32 KiB stages.  With them
@@ -24,7 +24,7 @@
 //
 // One CTA (768 threads; 384 without 4-bit weights), one role per warp:
 //   0       producer of the weights;  2  producer of the activations (one thread doing both was the limit of the ring)
-//   1       MMA issuer (leader only)
+//   1       MMA issuer (leader only); with packed activations warps 1 and 3 of the second CTA forward its converters' arrivals
 //   4-11    epilogue, two warps per TMEM lane quarter, alternating 32-token chunks; scales and problem fields are loaded
 //           one tile ahead (loading them per tile cost w8a8 8 x [4096, 2048, 1408] 20 us of 94)
 //   12-23   converters in three groups of four warps that take converted K blocks in turn (two groups: packed w4a4 and
@@ -32,10 +32,17 @@
 //
 // Barriers.  full[s] (leader): everything the MMAs of stage s read is in place in both CTAs - the loads of both (the
 // cta_group::2 form of a load completes on the leader's barrier) and, for converted weights, eight arrivals of converter
-// warps.  empty[s]: the MMAs of the stage have completed, committed to both CTAs; nothing else is needed, since they read
-// what the converters wrote from what the stage held.  wfull[n % kWBars]: this CTA's packed weights of converted K block n
-// have landed.  Every wait is bounded; a role whose wait runs out reports, raises the
-// CTA's abort flag and leaves its loop, the others follow by the flag or by their own limit.
+// warps, without release semantics: their payload is in tensor memory.  Packed activations are expanded into shared
+// memory, which a thread of the leader makes MMAs read: there the leader's converters release to full[s] at CTA scope,
+// those of the second CTA to their own xdone[s], and two otherwise idle warps pass that on to full[s] with a release at
+// cluster scope, which the issuer acquires.  That release takes some 2 000 cycles, now in the latency of a turn of the ring;
+// 8 x [4096, 2816, 2048], 8 x [4096, 2048, 1408], 60 x [24, 2816, 2048], us: no release at cluster scope (not sound)
+// 169 / 101 / 49, by the converters in their own chain 271 / 148 / 85, by two forwarders, one release for all stages that
+// are ready, 243 / 137 / 67, by one 272 / 151 / 69, by two with a release per stage 242 / 140 / 85.
+// empty[s]: the MMAs of the stage have completed, committed to both CTAs; nothing else is needed, since they read what the
+// converters wrote from what the stage held.  wfull[n % kWBars]: this CTA's packed weights of converted K block n have
+// landed.  Every wait is bounded; a role whose wait runs out reports, raises the CTA's abort flag and leaves its loop, the
+// others follow by the flag or by their own limit.
 #include "gg_tile.cuh"
 #include "launch.cuh"
 
@@ -81,6 +88,7 @@ struct CtrlD {
   uint64_t full[G::kStages];     // leader: all operands of the stage are in place in both CTAs (loads have landed, weights are converted)
   uint64_t wfull[G::kWBars];     // this CTA's packed weights (and packed activations) of converted K block n have landed: barrier n % kWBars
   uint64_t empty[G::kStages];    // the MMAs of the stage have completed (committed to both CTAs)
+  uint64_t xdone[G::kStages];    // second CTA: its converters have expanded the packed activations of the stage
   uint64_t tfull[2];             // accumulator b is complete (committed to both CTAs)
   uint64_t tempty[2];            // leader: both CTAs have drained accumulator b
   unsigned long long timeout_ns; // limit of every wait
@@ -104,13 +112,14 @@ constexpr uint32_t kCtrlOff = G::kRingBytes + G::kEpiBufs * kEpiStageS;   // Ctr
 #define MXB_CTRL(field) (kCtrlOff<G> + (uint32_t)offsetof(CtrlD<G>, field))
 
 // Bounded wait.  Everything it needs besides the barrier is in shared memory at a fixed distance from `sb`, so that a
-// role carries one register for all its waits.
-template <typename G>
+// role carries one register for all its waits.  kAcquire: see mbar_try_wait_cluster.
+template <typename G, bool kAcquire = false>
 __device__ __forceinline__ bool bar_wait(uint32_t sb, uint32_t bar, uint32_t parity) {
-  if (mbar_try_wait(bar, parity)) return true;
+  auto done = [&] { return kAcquire ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
+  if (done()) return true;
   const uint64_t t0 = globaltimer_ns();
   for (uint32_t it = 1;; ++it) {
-    if (mbar_try_wait(bar, parity)) return true;
+    if (done()) return true;
     if ((it & 63u) == 0) {
       if (lds32(sb + MXB_CTRL(abort_flag))) return false;
       if ((long long)(globaltimer_ns() - t0) > (long long)lds64(sb + MXB_CTRL(timeout_ns))) {
@@ -121,9 +130,9 @@ __device__ __forceinline__ bool bar_wait(uint32_t sb, uint32_t bar, uint32_t par
   }
 }
 // The whole warp polls (one instruction for the 32 lanes).
-template <typename G>
+template <typename G, bool kAcquire = false>
 __device__ __forceinline__ bool wwait(uint32_t sb, uint32_t bar, uint32_t parity) {
-  return __all_sync(0xffffffffu, bar_wait<G>(sb, bar, parity));
+  return __all_sync(0xffffffffu, bar_wait<G, kAcquire>(sb, bar, parity));
 }
 
 // tcgen05 N of a tile: the M = 256 form takes multiples of 32
@@ -137,7 +146,8 @@ struct MmaPos {
   bool ready;      // stage `stage` was seen complete already
 };
 
-template <int kV, typename G>
+// kAcquire: converters of both CTAs wrote an operand of the tile to shared memory (packed activations)
+template <int kV, bool kAcquire, typename G>
 __device__ __forceinline__ bool mma_tile(int nkb, MmaPos<G>& c, uint32_t smem_base, uint32_t d_tmem, uint32_t a0_tmem, uint32_t idesc) {
   const uint64_t desc0   = smem_desc_sw128(smem_base);
   const uint32_t desc_hi = (uint32_t)(desc0 >> 32);
@@ -145,11 +155,12 @@ __device__ __forceinline__ bool mma_tile(int nkb, MmaPos<G>& c, uint32_t smem_ba
   const uint32_t full0 = smem_base + MXB_CTRL(full), empty0 = smem_base + MXB_CTRL(empty);
   for (int kb = 0; kb < nkb; ++kb) {
     const int s = c.stage;
-    if (!c.ready && !wwait<G>(smem_base, full0 + 8 * s, c.phase)) return false;
+    if (!c.ready && !wwait<G, kAcquire>(smem_base, full0 + 8 * s, c.phase)) return false;
     if (++c.stage == G::kStages) { c.stage = 0; c.phase ^= 1u; }
     // the next stage's barrier is looked at before this stage's MMAs are issued: the round trip of the poll to shared
     // memory then overlaps the issue (test_wait: try_wait could suspend the warp)
-    const bool peek = mbar_test_wait(full0 + 8 * c.stage, c.phase);
+    const uint32_t nbar = full0 + 8 * c.stage;
+    const bool peek     = kAcquire ? mbar_test_wait_cluster(nbar, c.phase) : mbar_test_wait(nbar, c.phase);
     tc_fence_after_sync();
     const uint32_t wlo = w0 + s * (G::kStageBytes >> 4);
     if (elect_one_sync())
@@ -197,6 +208,8 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       mbar_init(smem_u32(&ctrl->empty[s]), 1);
     }
     for (int n = 0; n < G::kWBars; ++n) mbar_init(smem_u32(&ctrl->wfull[n]), 1);
+    if (kMode == 2)
+      for (int s = 0; s < G::kStages; ++s) mbar_init(smem_u32(&ctrl->xdone[s]), kCvtGroup);
     for (int b = 0; b < 2; ++b) {
       mbar_init(smem_u32(&ctrl->tfull[b]), 1);
       mbar_init(smem_u32(&ctrl->tempty[b]), 2 * kEpiWarps);
@@ -228,6 +241,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
   const int skip_stage     = blockIdx.x == 0 ? status->skip_stage - 1 : -1;   // test hook, see GGStatus
   const uint32_t tmem_base = ctrl->tmem_base;
   const uint32_t full0 = smem_base + MXB_CTRL(full), wfull0 = smem_base + MXB_CTRL(wfull), empty0 = smem_base + MXB_CTRL(empty);
+  const uint32_t xdone0 = smem_base + MXB_CTRL(xdone);
 
   // ------------------------------------------------------------------ roles
   if (warp == 0) {
@@ -328,6 +342,49 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         }
       }
     }
+  } else if (kMode == 2 && rank == 1 && (warp == 1 || warp == 3)) {
+    // ===== forwarders: warp 1 the even stages, warp 3 the odd ones (each barrier has one waiter, which sees all its phases) =====
+    if (elect_one_sync()) {
+      int stage = 0, i = -1, kb = 0, nkb = 0;
+      // this warp's next stage with packed activations, -1 at the end
+      auto next_stage = [&]() -> int {
+        for (;;) {
+          while (kb == nkb) {
+            if (++i >= my_tiles) return -1;
+            const TileS ti = decode_rec(tile_rec(i));
+            kb  = 0;
+            nkb = ti.nkb;
+            if (ti.scheme != SCH_W4A4) {
+              stage = (stage + nkb) % G::kStages;
+              kb    = nkb;
+            }
+          }
+          const int s = stage;
+          ++kb;
+          if (++stage == G::kStages) stage = 0;
+          if ((s & 1) == (warp >> 1)) return s;
+        }
+      };
+      uint32_t parities = 0;   // of the next use of every stage's barrier
+      int s = next_stage();
+      while (s >= 0) {
+        if (!bar_wait<G>(smem_base, xdone0 + 8 * s, (parities >> s) & 1u)) {
+          report_s(status, 5, cta + i * nctas);
+          break;
+        }
+        // one release for all stages that are ready by now
+        uint32_t ready = 0;
+        do {
+          ready |= 1u << s;
+          parities ^= 1u << s;
+          s = next_stage();
+        } while (s >= 0 && !((ready >> s) & 1u) && mbar_test_wait(xdone0 + 8 * s, (parities >> s) & 1u));
+        tc_fence_after_sync();
+        tc_fence_before_sync();
+        fence_acq_rel_cluster();
+        for (; ready; ready &= ready - 1) mbar_arrive_leader_relaxed_n(full0 + 8 * (__ffs(ready) - 1), kCvtGroup);
+      }
+    }
   } else if (warp == 1) {
     // ===== MMA issuer: the leader's warp 1 issues for both CTAs =====
     if (rank == 0) {
@@ -350,11 +407,11 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         const uint32_t idesc  = is_int ? idesc_i8(2 * kWT, npad) : idesc_f16(2 * kWT, npad);
         bool ok;
         if (!convert)
-          ok = is_int ? mma_tile<0, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc)
-                      : mma_tile<1, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc);
+          ok = is_int ? mma_tile<0, kMode == 2, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc)
+                      : mma_tile<1, kMode == 2, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc);
         else
-          ok = is_int ? mma_tile<2, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc)
-                      : mma_tile<3, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc);
+          ok = is_int ? mma_tile<2, kMode == 2, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc)
+                      : mma_tile<3, kMode == 2, G>(ti.nkb, pos, smem_base, d_tmem, a_tmem, idesc);
         if (!ok) {
           if (lane == 0) report_s(status, 3, cta + i * nctas);
           break;
@@ -670,7 +727,11 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         tmem_st_wait();
         tc_fence_before_sync();
         __syncwarp();
-        if (lane == 0) mbar_arrive_leader_relaxed(full0 + 8 * s);
+        if (lane == 0) {
+          // expanded activations lie in shared memory: release them, in the second CTA to its forwarders
+          if (kMode == 2 && ti.scheme == SCH_W4A4) mbar_arrive((rank == 0 ? full0 : xdone0) + 8 * s);
+          else                                     mbar_arrive_leader_relaxed(full0 + 8 * s);
+        }
         s += kCvtGroups;
         if (s >= G::kStages) s -= G::kStages;
         wb += kCvtGroups;

@@ -54,3 +54,21 @@ def test_the_kernels_have_this_arrangement():
     assert re.search(r"kWBars\s*= \(kStages \+ kCvtGroups - 1\) / kCvtGroups \* kCvtGroups;", duo)
     assert re.search(r"kWBars\s*= 2 \* kStages;", swap) and re.search(r"kCvtWarps\s*= 8;", swap)
     assert "wfull[G::kWBars]" in duo and "wfull[G::kWBars]" in swap
+
+
+def test_arrivals_release_what_converters_write_to_shared_memory():
+    """The CTA-pair kernel's converters signal the leader's MMA warp.  Without release semantics that is good for payloads in
+    tensor memory only.  Packed activations are expanded into shared memory: the leader's converters release to their own
+    barrier, the second CTA's to theirs, from which forwarders release at cluster scope, and the MMA warp acquires at it, by
+    the poll that looks ahead too."""
+    duo = (CSRC / "gg_duo_kernel.cu").read_text()
+    cvt = duo[duo.index("if (kMode == 2 && ti.scheme == SCH_W4A4) {"):]
+    cvt = cvt[:cvt.index("s += kCvtGroups;")]
+    assert cvt.index("convert_w4a4<") < cvt.index("fence_proxy_async_smem();") < cvt.index("__syncwarp();")
+    assert re.search(r"if \(kMode == 2 && ti\.scheme == SCH_W4A4\)\s+mbar_arrive\(\(rank == 0 \? full0 : xdone0\) \+ 8 \* s\);", cvt)
+    fwd = duo[duo.index("// ===== forwarders"):duo.index("// ===== MMA issuer")]
+    assert fwd.index("bar_wait<G>(smem_base, xdone0") < fwd.index("fence_acq_rel_cluster();") < fwd.index("mbar_arrive_leader_relaxed_n(full0")
+    mma = duo[duo.index("__device__ __forceinline__ bool mma_tile("):]
+    mma = mma[:mma.index("return true;")]
+    assert "wwait<G, kAcquire>(" in mma and "mbar_test_wait_cluster(" in mma
+    assert re.findall(r"mma_tile<(\d), ([^,]+), G>", duo) == [(str(v), "kMode == 2") for v in range(4)]

@@ -1,10 +1,12 @@
 """Mixed-precision decode layers replayed back to back: thousands of launches whose weight loads land out of order (several
 layers, a gigabyte of weights: more than the caches and address translations hold) must all give the first launch's bits."""
+import numpy as np
 import pytest
 import torch
 
-from mxmoe_b200 import workload
+from mxmoe_b200 import gg, workload
 from mxmoe_b200.layer import MoELayer
+from tests import util
 
 pytestmark = pytest.mark.gpu
 
@@ -32,3 +34,22 @@ def test_replays_give_the_same_bits(cuda_device, family, tokens):
         for layer, x, ids, w, first in layers:
             assert torch.equal(layer.forward_graph(x, ids, w), first)
             layer.check()
+
+
+@pytest.mark.parametrize("rows", [(23, 1, 32, 17, 8, 31), (200, 33, 385, 96, 191, 64)], ids=["short-tiles", "long-tiles"])
+def test_packed_activations_replay_bit_exact(cuda_device, rows):
+    """Packed 4-bit activations are expanded into shared memory by threads of both CTAs of a pair and read by MMAs that one
+    thread of the first CTA issues: every one of many launches gives the oracle's bits."""
+    rng = np.random.default_rng(len(rows) + rows[0])
+    cases = [util.WxAxCase(rng, m, n, 1408, 4) for m, n in zip(rows, (768, 640, 512, 1024, 384, 896))]
+    g = gg.GroupedGemm([c.problem(cuda_device) for c in cases])
+    want = [torch.from_numpy(c.ref.view(np.int16).copy()).to(cuda_device) for c in cases]
+    wrong = torch.zeros((), dtype=torch.int64, device=cuda_device)
+    for _ in range(300):
+        for c in cases:
+            c.C.fill_(float("nan"))
+        g.run(kernel="swap2")
+        for c, w in zip(cases, want):
+            wrong += (c.C.view(torch.int16) != w).sum()
+    g.check()
+    assert int(wrong) == 0
