@@ -75,6 +75,7 @@ struct DuoGeo {
   // Barriers of converted K blocks: one per block in turn, not per stage.  A wait by parity is good only for a waiter that saw
   // the barrier's previous phase end, and loads land out of order: a barrier must belong to one converter group for good.
   static constexpr int kWBars      = (kStages + kCvtGroups - 1) / kCvtGroups * kCvtGroups;
+  static constexpr int kXBars      = kMode == 2 ? kStages : 1;   // barriers of expanded activations
   static constexpr uint32_t kACol0 = 2 * kTok;
   static constexpr int kThreads    = (kFirstCvt + (kMode ? kCvtGroups * kCvtGroup : 0)) * 32;
   static constexpr int kEpiChunks  = (kTok + 63) / 64;       // 32-token chunks of a tile one epilogue warp takes
@@ -88,7 +89,6 @@ struct CtrlD {
   uint64_t full[G::kStages];     // leader: all operands of the stage are in place in both CTAs (loads have landed, weights are converted)
   uint64_t wfull[G::kWBars];     // this CTA's packed weights (and packed activations) of converted K block n have landed: barrier n % kWBars
   uint64_t empty[G::kStages];    // the MMAs of the stage have completed (committed to both CTAs)
-  uint64_t xdone[G::kStages];    // second CTA: its converters have expanded the packed activations of the stage
   uint64_t tfull[2];             // accumulator b is complete (committed to both CTAs)
   uint64_t tempty[2];            // leader: both CTAs have drained accumulator b
   unsigned long long timeout_ns; // limit of every wait
@@ -99,6 +99,7 @@ struct CtrlD {
   Sched sched;
   alignas(16) __half sa_stage[kEpiWarps][G::kEpiChunks * 32];   // per epilogue warp: per-token scales of its chunks
   alignas(16) TileRec recs[kDuoRecs];
+  uint64_t xdone[G::kXBars];     // second CTA: its converters have expanded the packed activations of the stage
 };
 
 template <typename G>
@@ -115,11 +116,10 @@ constexpr uint32_t kCtrlOff = G::kRingBytes + G::kEpiBufs * kEpiStageS;   // Ctr
 // role carries one register for all its waits.  kAcquire: see mbar_try_wait_cluster.
 template <typename G, bool kAcquire = false>
 __device__ __forceinline__ bool bar_wait(uint32_t sb, uint32_t bar, uint32_t parity) {
-  auto done = [&] { return kAcquire ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
-  if (done()) return true;
+  if (kAcquire ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
   const uint64_t t0 = globaltimer_ns();
   for (uint32_t it = 1;; ++it) {
-    if (done()) return true;
+    if (kAcquire ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)) return true;
     if ((it & 63u) == 0) {
       if (lds32(sb + MXB_CTRL(abort_flag))) return false;
       if ((long long)(globaltimer_ns() - t0) > (long long)lds64(sb + MXB_CTRL(timeout_ns))) {
@@ -159,8 +159,7 @@ __device__ __forceinline__ bool mma_tile(int nkb, MmaPos<G>& c, uint32_t smem_ba
     if (++c.stage == G::kStages) { c.stage = 0; c.phase ^= 1u; }
     // the next stage's barrier is looked at before this stage's MMAs are issued: the round trip of the poll to shared
     // memory then overlaps the issue (test_wait: try_wait could suspend the warp)
-    const uint32_t nbar = full0 + 8 * c.stage;
-    const bool peek     = kAcquire ? mbar_test_wait_cluster(nbar, c.phase) : mbar_test_wait(nbar, c.phase);
+    const bool peek = kAcquire ? mbar_test_wait_cluster(full0 + 8 * c.stage, c.phase) : mbar_test_wait(full0 + 8 * c.stage, c.phase);
     tc_fence_after_sync();
     const uint32_t wlo = w0 + s * (G::kStageBytes >> 4);
     if (elect_one_sync())
@@ -170,6 +169,53 @@ __device__ __forceinline__ bool mma_tile(int nkb, MmaPos<G>& c, uint32_t smem_ba
     if (kV >= 2) c.a = (c.a + 1) % G::kASlots;
   }
   return true;
+}
+
+// A forwarder (packed activations, second CTA): stages with s & 1 == odd, so that each xdone barrier has one waiter, which
+// sees all its phases.  One thread.
+template <typename G>
+__device__ __forceinline__ void forward_arrivals(const CtrlD<G>* ctrl, uint32_t smem_base, int count, int cta, int nctas, int my_tiles,
+                                                 int odd, GGStatus* status) {
+  const uint32_t full0 = smem_base + MXB_CTRL(full), xdone0 = smem_base + MXB_CTRL(xdone);
+  int stage = 0, i = -1, kb = 0, nkb = 0;
+  // the next of its stages that holds packed activations, -1 at the end
+  auto next_stage = [&]() -> int {
+    for (;;) {
+      while (kb == nkb) {
+        if (++i >= my_tiles) return -1;
+        const TileS ti = decode_rec(i < kDuoRecs ? ctrl->recs[i] : make_rec(&ctrl->sched, count, cta + i * nctas, G::kTok, G::kTok, 1));
+        kb  = 0;
+        nkb = ti.nkb;
+        if (ti.scheme != SCH_W4A4) {
+          stage = (stage + nkb) % G::kStages;
+          kb    = nkb;
+        }
+      }
+      const int s = stage;
+      ++kb;
+      if (++stage == G::kStages) stage = 0;
+      if ((s & 1) == odd) return s;
+    }
+  };
+  uint32_t parities = 0;   // of the next use of every stage's barrier
+  int s = next_stage();
+  while (s >= 0) {
+    if (!bar_wait<G>(smem_base, xdone0 + 8 * s, (parities >> s) & 1u)) {
+      report_s(status, 5, cta + i * nctas);
+      break;
+    }
+    // one release for all stages that are ready by now
+    uint32_t ready = 0;
+    do {
+      ready |= 1u << s;
+      parities ^= 1u << s;
+      s = next_stage();
+    } while (s >= 0 && !((ready >> s) & 1u) && mbar_test_wait(xdone0 + 8 * s, (parities >> s) & 1u));
+    tc_fence_after_sync();
+    tc_fence_before_sync();
+    fence_acq_rel_cluster();
+    for (; ready; ready &= ready - 1) mbar_arrive_leader_relaxed_n(full0 + 8 * (__ffs(ready) - 1), kCvtGroup);
+  }
 }
 
 }  // namespace
@@ -241,7 +287,6 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
   const int skip_stage     = blockIdx.x == 0 ? status->skip_stage - 1 : -1;   // test hook, see GGStatus
   const uint32_t tmem_base = ctrl->tmem_base;
   const uint32_t full0 = smem_base + MXB_CTRL(full), wfull0 = smem_base + MXB_CTRL(wfull), empty0 = smem_base + MXB_CTRL(empty);
-  const uint32_t xdone0 = smem_base + MXB_CTRL(xdone);
 
   // ------------------------------------------------------------------ roles
   if (warp == 0) {
@@ -343,47 +388,8 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       }
     }
   } else if (kMode == 2 && rank == 1 && (warp == 1 || warp == 3)) {
-    // ===== forwarders: warp 1 the even stages, warp 3 the odd ones (each barrier has one waiter, which sees all its phases) =====
-    if (elect_one_sync()) {
-      int stage = 0, i = -1, kb = 0, nkb = 0;
-      // this warp's next stage with packed activations, -1 at the end
-      auto next_stage = [&]() -> int {
-        for (;;) {
-          while (kb == nkb) {
-            if (++i >= my_tiles) return -1;
-            const TileS ti = decode_rec(tile_rec(i));
-            kb  = 0;
-            nkb = ti.nkb;
-            if (ti.scheme != SCH_W4A4) {
-              stage = (stage + nkb) % G::kStages;
-              kb    = nkb;
-            }
-          }
-          const int s = stage;
-          ++kb;
-          if (++stage == G::kStages) stage = 0;
-          if ((s & 1) == (warp >> 1)) return s;
-        }
-      };
-      uint32_t parities = 0;   // of the next use of every stage's barrier
-      int s = next_stage();
-      while (s >= 0) {
-        if (!bar_wait<G>(smem_base, xdone0 + 8 * s, (parities >> s) & 1u)) {
-          report_s(status, 5, cta + i * nctas);
-          break;
-        }
-        // one release for all stages that are ready by now
-        uint32_t ready = 0;
-        do {
-          ready |= 1u << s;
-          parities ^= 1u << s;
-          s = next_stage();
-        } while (s >= 0 && !((ready >> s) & 1u) && mbar_test_wait(xdone0 + 8 * s, (parities >> s) & 1u));
-        tc_fence_after_sync();
-        tc_fence_before_sync();
-        fence_acq_rel_cluster();
-        for (; ready; ready &= ready - 1) mbar_arrive_leader_relaxed_n(full0 + 8 * (__ffs(ready) - 1), kCvtGroup);
-      }
+    if constexpr (kMode == 2) {
+      if (elect_one_sync()) forward_arrivals<G>(ctrl, smem_base, count, cta, nctas, my_tiles, warp >> 1, status);
     }
   } else if (warp == 1) {
     // ===== MMA issuer: the leader's warp 1 issues for both CTAs =====
@@ -729,7 +735,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
         __syncwarp();
         if (lane == 0) {
           // expanded activations lie in shared memory: release them, in the second CTA to its forwarders
-          if (kMode == 2 && ti.scheme == SCH_W4A4) mbar_arrive((rank == 0 ? full0 : xdone0) + 8 * s);
+          if (kMode == 2 && ti.scheme == SCH_W4A4) mbar_arrive((rank == 0 ? full0 : smem_base + MXB_CTRL(xdone)) + 8 * s);
           else                                     mbar_arrive_leader_relaxed(full0 + 8 * s);
         }
         s += kCvtGroups;

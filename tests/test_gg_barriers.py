@@ -65,8 +65,8 @@ def test_arrivals_release_what_converters_write_to_shared_memory():
     cvt = duo[duo.index("if (kMode == 2 && ti.scheme == SCH_W4A4) {"):]
     cvt = cvt[:cvt.index("s += kCvtGroups;")]
     assert cvt.index("convert_w4a4<") < cvt.index("fence_proxy_async_smem();") < cvt.index("__syncwarp();")
-    assert re.search(r"if \(kMode == 2 && ti\.scheme == SCH_W4A4\)\s+mbar_arrive\(\(rank == 0 \? full0 : xdone0\) \+ 8 \* s\);", cvt)
-    fwd = duo[duo.index("// ===== forwarders"):duo.index("// ===== MMA issuer")]
+    assert re.search(r"if \(kMode == 2 && ti\.scheme == SCH_W4A4\)\s+mbar_arrive\(\(rank == 0 \? full0 : smem_base \+ MXB_CTRL\(xdone\)\) \+ 8 \* s\);", cvt)
+    fwd = duo[duo.index("void forward_arrivals("):duo.index("gg_duo_kernel(const")]
     assert fwd.index("bar_wait<G>(smem_base, xdone0") < fwd.index("fence_acq_rel_cluster();") < fwd.index("mbar_arrive_leader_relaxed_n(full0")
     mma = duo[duo.index("__device__ __forceinline__ bool mma_tile("):]
     mma = mma[:mma.index("return true;")]
