@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kBlock) quant_act_kernel(ActArgs a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row_in_blk = warp / kWarps, w = warp % kWarps;
   const int row     = blockIdx.x * (8 / kWarps) + row_in_blk;
-  const int live    = a.rows_dev ? min(a.rows_total, __ldg(a.rows_dev)) : a.rows_total;
+  const int live    = a.rows_dev ? min(a.rows_total, *a.rows_dev) : a.rows_total;
   if (blockIdx.x * (8 / kWarps) >= live) return;   // the whole block lies beyond the live rows
   const bool row_ok = row < live;
 
@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(kBlock) quant_act_kernel(ActArgs a) {
   for (int j = 0; j < kJ; ++j) {
     const int ci = chunk_of<kWarps>(w, j, lane);
     if (row_ok && ci < nchunk) {
-      unpack8(__ldg(reinterpret_cast<const uint4*>(src) + ci), x[j]);
+      unpack8(reinterpret_cast<const uint4*>(src)[ci], x[j]);
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[j][e] = 0.f;
@@ -435,7 +435,7 @@ __global__ void __launch_bounds__(kBlock, 3) quant_tokens_kernel(TokenQuantArgs 
   for (int j = 0; j < kJ; ++j) {
     const int ci = chunk_of<kWarps>(w, j, lane);
     if (row_ok && ci < nchunk) {
-      unpack8(__ldg(reinterpret_cast<const uint4*>(a.in + (int64_t)tok * a.k) + ci), x[j]);
+      unpack8(reinterpret_cast<const uint4*>(a.in + (int64_t)tok * a.k)[ci], x[j]);
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[j][e] = 0.f;
@@ -472,7 +472,7 @@ __global__ void __launch_bounds__(kBlock, 2) quant_tokens_scatter_kernel(TokenQu
   __half* s_base         = s_in_record ? r.q_store : r.s_store;
   int my_tag = -1, my_q = 0, my_s = -1;
   if (row_ok && lane < topk) {
-    const int row = __ldg(slot_row + (int64_t)tok * topk + lane);
+    const int row = slot_row[(int64_t)tok * topk + lane];
     if (row >= 0 && row < r.rows_routed) {
       const RowInfo ri = locate_row(r, row);
       my_tag = ri.tag;
@@ -485,7 +485,7 @@ __global__ void __launch_bounds__(kBlock, 2) quant_tokens_scatter_kernel(TokenQu
   for (int j = 0; j < kJ; ++j) {
     const int ci = chunk_of<kWarps>(w, j, lane);
     if (row_ok && ci < nchunk) {
-      unpack8(__ldg(reinterpret_cast<const uint4*>(a.in + (int64_t)tok * a.k) + ci), x[j]);
+      unpack8(reinterpret_cast<const uint4*>(a.in + (int64_t)tok * a.k)[ci], x[j]);
     } else {
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[j][e] = 0.f;
@@ -521,7 +521,7 @@ __global__ void __launch_bounds__(kBlock) gather_rows_kernel(ActArgs a, TokenQua
   const uint4* s = reinterpret_cast<const uint4*>(src + tok * (a.k / pack));
   uint4* d       = reinterpret_cast<uint4*>(ri.q_dst);
   const int n16  = (a.k / pack) >> 3;
-  for (int c = lane; c < n16; c += 32) d[c] = __ldg(s + c);
+  for (int c = lane; c < n16; c += 32) d[c] = s[c];
   if (ri.tag != 0 && lane == 0) *ri.s_dst = (ri.tag == 1 ? t.s8 : t.s4)[tok];
 }
 
@@ -538,7 +538,7 @@ __device__ __forceinline__ void rows_quant_body(const ActArgs& a) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row_in_blk = warp / kWarps, w = warp % kWarps;
   const int row     = blockIdx.x * (8 / kWarps) + row_in_blk;
-  const int live    = a.rows_dev ? min(a.rows_total, __ldg(a.rows_dev)) : a.rows_total;
+  const int live    = a.rows_dev ? min(a.rows_total, *a.rows_dev) : a.rows_total;
   if (blockIdx.x * (8 / kWarps) >= live) return;   // the whole block lies beyond the live rows
   const bool row_ok = row < live;
   RowInfo ri{0, 0, nullptr, nullptr};
@@ -560,8 +560,8 @@ __device__ __forceinline__ void rows_quant_body(const ActArgs& a) {
   for (int j = 0; j < kJ; ++j) {
     const int ci = chunk_of<kWarps>(w, j, lane);
     if (row_ok && ci < nchunk) {
-      gq[j] = __ldg(reinterpret_cast<const uint4*>(src) + ci);
-      if (kSilu) uq[j] = __ldg(reinterpret_cast<const uint4*>(src + ri.k) + ci);
+      gq[j] = reinterpret_cast<const uint4*>(src)[ci];
+      if (kSilu) uq[j] = reinterpret_cast<const uint4*>(src + ri.k)[ci];
     }
   }
 #pragma unroll

@@ -509,7 +509,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       for (int ch = half; ch < nchunk; ch += 2) {
         __syncwarp();   // the lanes left the previous chunk's stores one by one; tcgen05.ld takes the whole warp
         int64_t row_ptr = 0;
-        if (row_ptrs && lane < 8 && ch * 32 + q * 8 + lane < ntok) row_ptr = __ldg(row_ptrs + crow0 + ch * 32 + q * 8 + lane);
+        if (row_ptrs && lane < 8 && ch * 32 + q * 8 + lane < ntok) row_ptr = row_ptrs[crow0 + ch * 32 + q * 8 + lane];
         uint32_t v[32];
         tmem_ld_32x32(taddr + ch * 32, v);
         tmem_ld_wait();

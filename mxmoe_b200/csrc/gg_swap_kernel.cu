@@ -476,7 +476,7 @@ gg_swap_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatu
         __syncwarp();   // (tcgen05.ld takes the whole warp)
         // row-wide stores to per-row addresses: this lane's row of the chunk, fetched before the accumulator load
         int64_t row_ptr = 0;
-        if (row_ptrs && lane < 8 && ch * 32 + q * 8 + lane < ntok) row_ptr = __ldg(row_ptrs + crow0 + ch * 32 + q * 8 + lane);
+        if (row_ptrs && lane < 8 && ch * 32 + q * 8 + lane < ntok) row_ptr = row_ptrs[crow0 + ch * 32 + q * 8 + lane];
         uint32_t v[32];
         tmem_ld_32x32(taddr + ch * 32, v);
         tmem_ld_wait();

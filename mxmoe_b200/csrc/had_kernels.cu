@@ -37,9 +37,8 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], const uint32_t (&a)[4],
 
 // KP: K rounded up to a multiple of 16 (rows and columns beyond K are zero)
 template <int KP, bool kFwht8>
-__global__ void __launch_bounds__(kThreads) had_kron_kernel(const __half* __restrict__ in, __half* __restrict__ out,
-                                                            const __half* __restrict__ hadK, int rows, int K, int m,
-                                                            float scale) {
+__global__ void __launch_bounds__(kThreads) had_kron_kernel(const __half* in, __half* out, const __half* __restrict__ hadK,
+                                                            int rows, int K, int m, float scale) {
   release_dependents();
   grid_dependency_wait();
   constexpr int LD = KP + 8;                         // row pitch of both shared tiles (halfs): keeps ldmatrix conflict-free

@@ -10,6 +10,10 @@
 //   * all threads call grid_dependency_wait() before the first access to memory that any kernel reads or writes (only
 //     the status block of a problem list, which a copy wrote before the chain began, is read earlier).  A kernel
 //     therefore ends after all of its predecessors, and whatever follows it in the stream in the ordinary way does too.
+//   * What a kernel of the chain writes is read with ordinary loads: no __ldg, no `const T* __restrict__` parameter.  Both
+//     promise data that stays constant for the whole life of the reading kernel; its blocks are resident while their
+//     predecessor still writes, and such loads may be moved above the wait.  Weights, their scales, sign vectors, Hadamard
+//     factors and problem lists are constant and may be read that way.
 //   * release_dependents() comes first: it only lets the next kernel's blocks become resident, and since that happens
 //     when the LAST block has called it, no waiting block takes the place of one that still has to start.  The grouped
 //     GEMM does not call it: its launch fills every SM until it ends (with it, in graphs: 61 tokens mixed 146 -> 152 us,

@@ -185,9 +185,8 @@ __global__ void __launch_bounds__(kThreads) route_scatter_kernel(RouteArgs a) {
 }
 
 // out[t] = sum_j w[t,j] * y[slot_row[t,j]] (+ y_shared[t]); fp32 accumulation, fp16 result
-__global__ void __launch_bounds__(kThreads) combine_kernel(const __half* __restrict__ y, const int* __restrict__ slot_row,
-                                                           const float* __restrict__ w, const __half* __restrict__ ysh,
-                                                           __half* __restrict__ out, int topk, int hidden) {
+__global__ void __launch_bounds__(kThreads) combine_kernel(const __half* y, const int* slot_row, const float* w,
+                                                           const __half* ysh, __half* out, int topk, int hidden) {
   release_dependents();
   grid_dependency_wait();
   const int t = blockIdx.x;
@@ -199,7 +198,7 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const __half* __restr
       const int r = slot_row[t * topk + j];
       if (r < 0) continue;
       const float wt = w ? w[t * topk + j] : 1.f;
-      const uint4 v  = __ldg(reinterpret_cast<const uint4*>(y + (int64_t)r * hidden) + c);
+      const uint4 v  = reinterpret_cast<const uint4*>(y + (int64_t)r * hidden)[c];
       const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -209,7 +208,7 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const __half* __restr
       }
     }
     if (ysh) {
-      const uint4 v = __ldg(reinterpret_cast<const uint4*>(ysh + (int64_t)t * hidden) + c);
+      const uint4 v = reinterpret_cast<const uint4*>(ysh + (int64_t)t * hidden)[c];
       const __half2* h = reinterpret_cast<const __half2*>(&v);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
@@ -230,8 +229,8 @@ __global__ void __launch_bounds__(kThreads) combine_kernel(const __half* __restr
 // optionally renormalised to sum 1 (the gate of the MoE blocks the reference quantises: softmax -> topk ->
 // norm_topk_prob).  One warp per token, up to 16 experts per lane; ties go to the lower expert index.
 template <typename T>
-__global__ void __launch_bounds__(kThreads) gate_topk_kernel(const T* __restrict__ logits, int num_tokens, int E, int topk,
-                                                             int renorm, int* __restrict__ ids, float* __restrict__ wts) {
+__global__ void __launch_bounds__(kThreads) gate_topk_kernel(const T* logits, int num_tokens, int E, int topk,
+                                                             int renorm, int* ids, float* wts) {
   release_dependents();
   grid_dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

@@ -4,7 +4,7 @@ import numpy as np
 import pytest
 import torch
 
-from mxmoe_b200 import gg, workload
+from mxmoe_b200 import gg, ops, workload
 from mxmoe_b200.layer import MoELayer
 from tests import util
 
@@ -52,4 +52,37 @@ def test_packed_activations_replay_bit_exact(cuda_device, rows):
         for c, w in zip(cases, want):
             wrong += (c.C.view(torch.int16) != w).sum()
     g.check()
+    assert int(wrong) == 0
+
+
+@pytest.mark.parametrize("side_stream", [False, True])
+def test_eager_chain_with_changing_inputs(cuda_device, side_stream):
+    """Launches of the chain overlap: every step of an eager loop over two inputs and routings, whose buffers all steps share,
+    gives the bits of that input alone, with nothing between the steps that would separate them."""
+    spec = workload.LayerSpec("tiny", 12, 3, 1024, 768, 768, 150, "zipf", 1.2, True, True, "mixed5")
+    gu, dn, signs, _ = workload.build_layer_weights(spec, gen_device=cuda_device, device=cuda_device)
+    layer = MoELayer(spec.num_experts, spec.topk, spec.hidden, spec.inter, gu, dn, spec.tokens,
+                     shared_inter=spec.shared_inter, signs=signs, rotate=spec.rotate, device=cuda_device)
+    inputs, want = [], []
+    for seed in range(2):
+        gen = torch.Generator(device=cuda_device).manual_seed(seed)
+        x = workload.make_hidden(spec, seed=seed, device=cuda_device)
+        logits = torch.randn(spec.tokens, spec.num_experts, generator=gen, device=cuda_device)
+        inputs.append((x, logits))
+        ids, w = ops.gate_topk(logits, spec.topk)
+        want.append(layer.forward(x, ids, w).clone())
+        torch.cuda.synchronize()
+    assert not torch.equal(want[0], want[1])
+    stream = torch.cuda.Stream() if side_stream else torch.cuda.current_stream()
+    wrong = torch.zeros((), dtype=torch.int64, device=cuda_device)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        for step in range(400):
+            for i in (step & 1, 1 - (step & 1)):
+                ids, w = ops.gate_topk(inputs[i][1], spec.topk)
+                out = layer.forward(inputs[i][0], ids, w)
+                if step % 4 == 0:      # otherwise the next step follows at once
+                    wrong += (out.view(torch.int16) != want[i].view(torch.int16)).sum()
+    torch.cuda.synchronize()
+    layer.check()
     assert int(wrong) == 0
