@@ -2,9 +2,9 @@
 //
 // The kernels of a layer form a chain, each reading what the one before wrote.  With a plain launch the next kernel's
 // blocks are scheduled only after the last block of the previous one has ended and its writes are flushed.  Launched
-// through launch_dependent, a kernel's blocks become resident as soon as every block of the previous kernel has begun
-// (and SM resources allow), set up what depends on no earlier kernel and wait in grid_dependency_wait() for the previous
-// kernel to have completed with its writes visible.
+// through launch_dependent, a kernel's blocks become resident as soon as every block of the previous kernel has released
+// it or ended (and SM resources allow), set up what depends on no earlier kernel and wait in grid_dependency_wait() for the
+// previous kernel to have completed with its writes visible.
 //
 // Rules that every kernel launched this way keeps:
 //   * all threads call grid_dependency_wait() before the first access to memory that any kernel reads or writes (only
@@ -15,16 +15,23 @@
 //     predecessor still writes, and such loads may be moved above the wait.  Weights, their scales, sign vectors, Hadamard
 //     factors and problem lists are constant and may be read that way.
 //   * release_dependents() comes first: it only lets the next kernel's blocks become resident, and since that happens
-//     when the LAST block has called it, no waiting block takes the place of one that still has to start.  The grouped
-//     GEMM does not call it: its launch fills every SM until it ends (with it, in graphs: 61 tokens mixed 146 -> 152 us,
-//     16 tokens of the mixtral shape 212 -> 219, 8192 tokens w4a4 436 -> 440).
-// Measured (us, before -> after): 500 tokens behind the gate 180.3 -> 168.4, 1 token 67.9 -> 66.6, 8192 tokens w4a4 436.5 -> 431.7.
+//     when the LAST block has called it, no waiting block takes the place of one that still has to start.  Launches of ONE
+//     block release early (the routing of a decode batch, the quantisers and the combine of a few tokens): the next
+//     kernel's blocks set up on the SMs that stay idle.  Larger launches release when they end: blocks that wait beside
+//     running ones cost more than their set-up takes.  Graphs and eager steps, us, everyone releases early / one block
+//     only / nobody / plain launches: 500 tokens behind the gate 168.4 / 155.0 / 155.6 / 178.8, 1009 tokens fp16 251.3 /
+//     246.7 / 246.3 / 261.7, 61 tokens mixed 142.7 / 138.8 / 138.9 / 140.5, 16 tokens of the mixtral shape 200.5 / 198.0 /
+//     197.8 / 198.3, 1 token 63.6 / 63.6 / 65.5 / 64.7, 32 tokens 161.5 / 160.5 / 160.4 / 161.9, 8192 tokens w4a4 429.2 / 431.1 /
+//     430.6 / 431.4 (limits of 8 and 32 blocks: 61 tokens mixed 140.0 and 140.1).  The grouped GEMM fills every SM and
+//     never releases early.
 #pragma once
 #include <cuda_runtime.h>
 
 namespace mxb {
 
-__device__ __forceinline__ void release_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void release_dependents() {
+  if (gridDim.x == 1) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <typename... P, typename... A>
