@@ -431,9 +431,9 @@ int run_kernel(void* workspace, const mxmoe_gg_plan* plan, int kernel, int num_c
   if (kernel == GGK_PAIR && n < 2) kernel = GGK_SINGLE;
   if (kernel == GGK_SWAP2 && n < 2) kernel = GGK_SWAP;   // a pair needs two CTAs
   const bool ext = (plan->flags & 4) != 0;
-  if (kernel == GGK_SWAP2)      mxb::gg_launch_duo(swp, count, status, needs_cvt, (plan->flags & 2) != 0, ext, n & ~1, cs);
+  if (kernel == GGK_SWAP2)      CUDA_TRY(mxb::gg_launch_duo(swp, count, status, needs_cvt, (plan->flags & 2) != 0, ext, n & ~1, cs));
   else if (kernel == GGK_PAIR)  CUDA_TRY(mxb::gg_launch_pair(probs, count, status, needs_cvt, n & ~1, cs));
-  else if (kernel == GGK_SWAP)  mxb::gg_launch_swap(swp, count, status, needs_cvt, ext, n, cs);
+  else if (kernel == GGK_SWAP)  CUDA_TRY(mxb::gg_launch_swap(swp, count, status, needs_cvt, ext, n, cs));
   else                          mxb::gg_launch_single(probs, count, status, needs_cvt, n, cs);
   CUDA_TRY(cudaGetLastError());
   return MXMOE_OK;

@@ -781,16 +781,17 @@ cudaError_t configure_duo() {
   return cudaFuncSetAttribute(gg_duo_kernel<kMode, kShort, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytes);
 }
 template <int kMode, bool kShort>
-void launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
+cudaError_t launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
   using G = DuoGeo<kMode, kShort>;
-  launch_dependent(ext ? gg_duo_kernel<kMode, kShort, true> : gg_duo_kernel<kMode, kShort, false>, num_ctas & ~1, G::kThreads,
-                   smem_bytes_duo<G>(), stream, problems, count, status);
+  return launch_dependent(ext ? gg_duo_kernel<kMode, kShort, true> : gg_duo_kernel<kMode, kShort, false>, num_ctas & ~1, G::kThreads,
+                          smem_bytes_duo<G>(), stream, problems, count, status);
 }
 template <bool kShort>
-void launch_mode(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas, cudaStream_t stream) {
-  if (cvt_mode == 2)  launch_duo<2, kShort>(problems, count, status, ext, num_ctas, stream);
-  else if (cvt_mode)  launch_duo<1, kShort>(problems, count, status, ext, num_ctas, stream);
-  else                launch_duo<0, kShort>(problems, count, status, ext, num_ctas, stream);
+cudaError_t launch_mode(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
+                        cudaStream_t stream) {
+  if (cvt_mode == 2) return launch_duo<2, kShort>(problems, count, status, ext, num_ctas, stream);
+  if (cvt_mode)      return launch_duo<1, kShort>(problems, count, status, ext, num_ctas, stream);
+  return launch_duo<0, kShort>(problems, count, status, ext, num_ctas, stream);
 }
 }  // namespace
 
@@ -804,10 +805,10 @@ cudaError_t gg_configure_duo() {
   return configure_duo<2, true>();
 }
 
-void gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool short_tiles, bool ext,
-                   int num_ctas, cudaStream_t stream) {
-  if (short_tiles) launch_mode<true>(problems, count, status, cvt_mode, ext, num_ctas, stream);
-  else             launch_mode<false>(problems, count, status, cvt_mode, ext, num_ctas, stream);
+cudaError_t gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool short_tiles, bool ext,
+                          int num_ctas, cudaStream_t stream) {
+  return short_tiles ? launch_mode<true>(problems, count, status, cvt_mode, ext, num_ctas, stream)
+                     : launch_mode<false>(problems, count, status, cvt_mode, ext, num_ctas, stream);
 }
 
 }  // namespace mxb

@@ -767,9 +767,9 @@ cudaError_t configure_one() {
   return cudaFuncSetAttribute(gg_swap_kernel<kMode, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
 }
 template <int kMode>
-void launch_one(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
-  launch_dependent(ext ? gg_swap_kernel<kMode, true> : gg_swap_kernel<kMode, false>, num_ctas, CfgS<kMode>::kThreads, kSmemBytes,
-                   stream, problems, count, status);
+cudaError_t launch_one(const GGSwapProblemDev* problems, int count, GGStatus* status, bool ext, int num_ctas, cudaStream_t stream) {
+  return launch_dependent(ext ? gg_swap_kernel<kMode, true> : gg_swap_kernel<kMode, false>, num_ctas, CfgS<kMode>::kThreads,
+                          kSmemBytes, stream, problems, count, status);
 }
 }  // namespace
 
@@ -786,11 +786,11 @@ cudaError_t gg_configure_swap() {
   return configure_one<2>();
 }
 
-void gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
-                    cudaStream_t stream) {
-  if (cvt_mode == 2)  launch_one<2>(problems, count, status, ext, num_ctas, stream);
-  else if (cvt_mode)  launch_one<1>(problems, count, status, ext, num_ctas, stream);
-  else                launch_one<0>(problems, count, status, ext, num_ctas, stream);
+cudaError_t gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
+                           cudaStream_t stream) {
+  if (cvt_mode == 2) return launch_one<2>(problems, count, status, ext, num_ctas, stream);
+  if (cvt_mode)      return launch_one<1>(problems, count, status, ext, num_ctas, stream);
+  return launch_one<0>(problems, count, status, ext, num_ctas, stream);
 }
 
 }  // namespace mxb

@@ -126,12 +126,12 @@ cudaError_t gg_configure_pair();
 // kernel with swapped operands (gg_swap_kernel.cu): weights from tensor memory / shared memory as the M side,
 // token tiles of up to 176 rows as the N side
 // `ext`: the launch holds problems with an optional result form (weight maps of rank 4), see gg_swap_kernel
-void gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
-                    cudaStream_t stream);
+cudaError_t gg_launch_swap(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool ext, int num_ctas,
+                           cudaStream_t stream);
 cudaError_t gg_configure_swap();
 // CTA pairs (gg_duo_kernel.cu); num_ctas >= 2; `short_tiles`: token tiles of 32 rows
-void gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool short_tiles, bool ext,
-                   int num_ctas, cudaStream_t stream);
+cudaError_t gg_launch_duo(const GGSwapProblemDev* problems, int count, GGStatus* status, int cvt_mode, bool short_tiles, bool ext,
+                          int num_ctas, cudaStream_t stream);
 cudaError_t gg_configure_duo();
 
 }  // namespace mxb

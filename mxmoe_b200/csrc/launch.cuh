@@ -46,7 +46,9 @@ cudaError_t launch_dependent(void (*kernel)(P...), int grid, int threads, size_t
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs    = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+  if (e != cudaSuccess) cudaGetLastError();   // the caller reports e; a later launch's check must not find it again
+  return e;
 }
 
 }  // namespace mxb

@@ -1,6 +1,8 @@
 """Kernels launched with launch_dependent are resident while the kernel before them still writes: they may use read-only loads
 (__ldg, or parameters that are pointers to const with __restrict__) only for data no kernel of the chain writes."""
 import re
+import shutil
+import subprocess
 from pathlib import Path
 
 import pytest
@@ -56,3 +58,22 @@ def test_only_single_block_launches_release_early():
     text = re.sub(r"//[^\n]*", "", (CSRC / "launch.cuh").read_text())
     assert re.search(r"if \(gridDim\.x == 1\) asm volatile\(\"griddepcontrol\.launch_dependents;\"", text)
     assert sum(p.read_text().count("griddepcontrol.launch_dependents") for p in CSRC.iterdir()) == 1
+
+
+@pytest.mark.gpu
+@pytest.mark.skipif(shutil.which("nvcc") is None, reason="no nvcc")
+def test_a_refused_launch_is_reported_once(tmp_path):
+    """launch_dependent returns the error and leaves none behind for the next check of the runtime's last error (a block of 4096
+    threads is refused on the host)."""
+    (tmp_path / "t.cu").write_text('''
+#include "launch.cuh"
+__global__ void k(int) {}
+int main() {
+  const cudaError_t e = mxb::launch_dependent(k, 1, 4096, 0, (cudaStream_t)0, 0);
+  return (e != cudaSuccess && cudaPeekAtLastError() == cudaSuccess) ? 0 : 1;
+}
+''')
+    exe = tmp_path / "t"
+    subprocess.run(["nvcc", "-std=c++17", "-gencode", "arch=compute_100a,code=sm_100a", "-I", str(CSRC), "-o", str(exe),
+                    str(tmp_path / "t.cu")], check=True)
+    assert subprocess.run([str(exe)]).returncode == 0
