@@ -169,6 +169,7 @@ int mxmoe_gg_debug(void* workspace, int timeout_ms, int skip_stage, void* stream
  * `workspace`.  counters[16]: 0 kernel body, 1 producer waiting for a free stage, 2 MMA issuer waiting
  * for operands, 3 MMA issuer waiting for a drained accumulator, 4 MMA issue, 5 epilogue waiting,
  * 6 epilogue draining + storing, 7 converter waiting, 8 converter working, 9 tiles, 10 stages.
+ * SWAP2 (the default) records 0, 9 and 10; the others also record 1 to 8, SWAP in builds with -DMXMOE_PROF only.
  * Synchronises `stream`. */
 int mxmoe_gg_profile(void* workspace, uint64_t* counters, void* stream);
 

@@ -92,6 +92,7 @@ struct CtrlD {
   uint64_t tfull[2];             // accumulator b is complete (committed to both CTAs)
   uint64_t tempty[2];            // leader: both CTAs have drained accumulator b
   unsigned long long timeout_ns; // limit of every wait
+  long long t0;                  // clock when the first CTA began (PROF_TOTAL)
   uint32_t tmem_base;
   int abort_flag;
   int pad[4];                    // outcome of a group's wait for an accumulator (kExt)
@@ -261,6 +262,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
       mbar_init(smem_u32(&ctrl->tempty[b]), 2 * kEpiWarps);
     }
     ctrl->abort_flag = 0;
+    ctrl->t0         = clock64();
     ctrl->timeout_ns = status->timeout_ms > 0 ? (uint64_t)status->timeout_ms * 1000000ull : kTimeoutNs;
     fence_mbar_init();
   }
@@ -385,6 +387,10 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
           }
           if (++stage == G::kStages) { stage = 0; phase ^= 1u; }
         }
+      }
+      if (blockIdx.x == 0) {
+        status->prof[PROF_TILES]  = my_tiles;
+        status->prof[PROF_STAGES] = n_stage;
       }
     }
   } else if (kMode == 2 && rank == 1 && (warp == 1 || warp == 3)) {
@@ -758,6 +764,7 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
 
   // ---------------------------------------------------------------- teardown
   __syncthreads();
+  if (blockIdx.x == 0 && tid == 0) status->prof[PROF_TOTAL] = clock64() - ctrl->t0;
   if (*reinterpret_cast<volatile int*>(&ctrl->abort_flag)) {
     // give copies that are still in flight time to land before shared memory is released
     const uint64_t t0 = globaltimer_ns();

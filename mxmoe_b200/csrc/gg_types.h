@@ -85,7 +85,8 @@ struct alignas(256) GGStatus {
   int where;       // role << 24 | tile index
   int count;       // problems prepared
   int needs_cvt;   // any problem needs the converter warps
-  // cycle counters of CTA 0 of the last launch (clock64 deltas), see GGProf
+  // cycle counters of CTA 0 of the last launch (clock64 deltas), see GGProf; the kernel on CTA pairs fills the total, the
+  // tiles and the stages
   unsigned long long prof[16];
   int prof_on;      // per-role cycle counters wanted (costs a few percent)
   int timeout_ms;   // limit of every bounded wait of the kernel with swapped operands; 0 = 1000 ms

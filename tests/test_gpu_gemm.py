@@ -5,6 +5,8 @@ compared bit for bit.  Floating-point schemes (fp16, w4a16 group-128):
 rel-L2 <= 1e-3 against the oracle (fp64 accumulation rounded once), the bound the
 specification states for fp16 outputs.
 """
+import os
+
 import numpy as np
 import pytest
 import torch
@@ -314,3 +316,18 @@ def test_more_problems_than_one_launch_walks(cuda_device):
     assert g.kept == 257
     for i in (0, 100, 255, 256):
         assert np.array_equal(cases[i].C.cpu().numpy().view(np.uint16), cases[i].ref.view(np.uint16)), i
+
+
+def test_profile_counts_tiles_and_stages(cuda_device, gg_kernel):
+    """Every kernel reports cycles, tiles and pipeline stages of its first CTA (or pair): one CTA (pair) walks all tiles here."""
+    rng = np.random.default_rng(7)
+    c = util.WxAxCase(rng, 40, 512, 384, 8)          # K: three blocks of 128 bytes
+    g = gg.GroupedGemm([c.problem(cuda_device)])
+    g.run(num_ctas=2 if gg_kernel in ("swap2", "pair") else 1)
+    g.check()
+    p = gg.profile(g)
+    rows, channels = {"single": (128, 256), "pair": (256, 256), "swap": (176, 128), "swap2": (256, 256)}[gg_kernel]
+    if gg_kernel == "swap2" and os.environ.get("MXMOE_GG_TILES") == "small":
+        rows = 32
+    tiles = -(-40 // rows) * -(-512 // channels)
+    assert (p["tiles"], p["stages"]) == (tiles, 3 * tiles) and p["total"] > 0
