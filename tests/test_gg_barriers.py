@@ -54,6 +54,9 @@ def test_the_kernels_have_this_arrangement():
     assert re.search(r"kWBars\s*= \(kStages \+ kCvtGroups - 1\) / kCvtGroups \* kCvtGroups;", duo)
     assert re.search(r"kWBars\s*= 2 \* kStages;", swap) and re.search(r"kCvtWarps\s*= 8;", swap)
     assert "wfull[G::kWBars]" in duo and "wfull[G::kWBars]" in swap
+    # every role that walks these barriers wraps at their number, not at the ring's length
+    assert "if (++wbar == G::kWBars) wbar = 0;" in duo and duo.count("wb -= G::kWBars; wpar ^= 1u;") == 2
+    assert swap.count("if (++wb == G::kWBars) wb = 0;") == 2 and swap.count("if (++wb == G::kWBars) { wb = 0; wphase ^= 1u; }") >= 1
 
 
 def test_arrivals_release_what_converters_write_to_shared_memory():

@@ -17,10 +17,11 @@ from tests import util
 pytestmark = pytest.mark.gpu
 
 
-@pytest.fixture(autouse=True, params=["swap", "swap-small"])
+@pytest.fixture(autouse=True, params=["swap", "swap2", "swap2-small"])
 def gg_tiles(request, monkeypatch):
-    monkeypatch.setenv("MXMOE_GG_KERNEL", "swap")
-    if request.param == "swap-small":
+    """Both kernels that have this epilogue; "swap2-small": 32-row token tiles of the kernel on CTA pairs on every shape."""
+    monkeypatch.setenv("MXMOE_GG_KERNEL", request.param.split("-")[0])
+    if request.param.endswith("-small"):
         monkeypatch.setenv("MXMOE_GG_TILES", "small")
     else:
         monkeypatch.delenv("MXMOE_GG_TILES", raising=False)
@@ -110,7 +111,7 @@ def _layers(spec, dev, **kw):
 
 @pytest.mark.parametrize("scheme,shared", [("w4a4_g-1_sym", False), ("w8a8_g-1_sym", True), ("fp16", False)])
 def test_layer_with_fused_silu_equals_layer_without(cuda_device, scheme, shared, gg_tiles):
-    if gg_tiles != "swap":
+    if gg_tiles.endswith("-small"):
         pytest.skip("layers choose their own tile geometry")
     spec = workload.LayerSpec("tiny", 6, 2, 512, 256, 512 if shared else 0, 70, "zipf", 1.2, True,
                               scheme != "fp16", scheme)
@@ -134,7 +135,7 @@ def test_layer_with_fused_silu_equals_layer_without(cuda_device, scheme, shared,
 
 
 def test_weight_only_layer_keeps_the_two_step_path(cuda_device, gg_tiles):
-    if gg_tiles != "swap":
+    if gg_tiles.endswith("-small"):
         pytest.skip("layers choose their own tile geometry")
     spec = workload.LayerSpec("tiny", 6, 2, 512, 256, 0, 40, "zipf", 1.2, True, False, "w4a16_g128_asym")
     fused, _ = _layers(spec, cuda_device)

@@ -2,9 +2,10 @@
 workspace usable.
 
 Every mbarrier wait of the grouped GEMM is bounded (1 s by default).  The failure is produced on the host: a test
-hook of the C ABI (mxmoe_gg_debug) shortens the limit to 20 ms and tells the producer of CTA 0 to leave out one
-weight load, so the barrier that load would complete is a flag that nothing sets.  Nothing traps, faults or spins
-without a limit; the other CTAs finish their tiles normally.
+hook of the C ABI (mxmoe_gg_debug) shortens the limit to 20 ms and tells the producer of CTA 0 to announce more bytes
+for one stage than it loads, so the barrier of that stage is a flag that nothing sets.  On a CTA pair the other CTA of the
+pair waits for the same accumulator and runs into its own limit.  Nothing traps, faults or spins without a limit; the other
+CTAs finish their tiles normally.
 """
 import time
 
@@ -19,18 +20,23 @@ from tests import util
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("bits,expanded", [(4, True), (8, False)])
-def test_wait_runs_out_then_workspace_recovers(cuda_device, bits, expanded):
+# the kernel on CTA pairs (the default) with long and with 32-row token tiles, and the single-CTA form; 4-bit weights alone, packed
+# activations as well (expanded=False), nothing to convert
+@pytest.mark.parametrize("kernel,rows,bits,expanded", [
+    ("swap", 300, 4, True), ("swap", 300, 8, False),
+    ("swap2", 300, 4, True), ("swap2", 300, 4, False), ("swap2", 300, 8, False),
+    ("swap2", 24, 4, True), ("swap2", 24, 4, False), ("swap2", 24, 8, False)])
+def test_wait_runs_out_then_workspace_recovers(cuda_device, bits, expanded, kernel, rows):
     rng = np.random.default_rng(bits)
-    c = util.WxAxCase(rng, 300, 512, 512, bits, expanded=expanded)     # CTA 0 owns tile 0: four pipeline stages
+    c = util.WxAxCase(rng, rows, 512, 512, bits, expanded=expanded)    # CTA 0 (its pair) owns tile 0: four pipeline stages
     g = gg.GroupedGemm([c.problem(cuda_device)])
-    g.run(kernel="swap")
+    g.run(kernel=kernel)
     g.check()
     assert np.array_equal(c.C.cpu().numpy().view(np.uint16), c.ref.view(np.uint16))
 
     g.debug(timeout_ms=20, skip_stage=2)
     t0 = time.time()
-    g.run(kernel="swap")
+    g.run(kernel=kernel)
     with pytest.raises(MxMoEError) as err:
         g.check()
     elapsed = time.time() - t0
@@ -45,6 +51,6 @@ def test_wait_runs_out_then_workspace_recovers(cuda_device, bits, expanded):
     # the report was taken and cleared: the same workspace runs again, bit-exact
     g.debug(timeout_ms=0, skip_stage=-1)
     c.C.fill_(float("nan"))
-    g.run(kernel="swap")
+    g.run(kernel=kernel)
     g.check()
     assert np.array_equal(c.C.cpu().numpy().view(np.uint16), c.ref.view(np.uint16))
