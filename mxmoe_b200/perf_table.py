@@ -11,9 +11,9 @@ scheme the persistent kernel is timed on grouped launches whose tile count sweep
 of one wave to many waves at fixed N and K, and ``time = first_iter_cost + inc * tiles`` is fitted
 by least squares over the multi-wave points; ``stderr`` is the residual standard deviation.  The key
 is the ``repr`` of a dataclass with the reference's field names (``tile_config.py:195-207``), so the
-file drops into the solver unchanged; B200 has one tile shape per scheme (up to 176 token rows x 128
-output channels, 128 bytes of K per stage: the kernel with swapped operands; w4a4 is profiled with the
-layer's expanded int4 activations).
+file drops into the solver unchanged; B200 has one tile shape per scheme, that of the default kernel, which works on CTA
+pairs (256 output channels x up to 256 token rows, 192 with 4-bit weights; 128 bytes of K per stage).  Each scheme is
+profiled in launches of its own, w4a4 with the layer's expanded int4 activations.
 
     python -m mxmoe_b200.perf_table [out.json]
 """
@@ -51,37 +51,46 @@ class QConfig:
 
 @dataclasses.dataclass
 class TileConfig:
-    BM: int = 176
-    BN: int = 128
+    BM: int = 256
+    BN: int = 256
     BK: int = 128
     WM: int = 4
     WN: int = 1
     WK: int = 1
-    STAGE: int = 5
+    STAGE: int = 6
     SPLITK: int = -1
     MMA: str = "TCGEN05_F16_F32"
     QCFGA: object = dataclasses.field(default_factory=NO_QUANT)
     QCFGB: object = dataclasses.field(default_factory=NO_QUANT)
 
 
+# The tile of the default kernel (constants of csrc/gg_types.h and csrc/gg_duo_kernel.cu): output channels, and token rows
+# and pipeline stages without / with 4-bit weights in the launch.
+CHANNELS = 256
+TOKENS, STAGES = 256, 6
+TOKENS_4BIT, STAGES_4BIT = 192, 7
+
+
 def b200_tile(scheme: str) -> TileConfig:
     """The tile the sm_100a kernel uses for ``scheme`` (BK in elements of K per pipeline stage)."""
     from .weights import parse_scheme
     a, w, g, sym = parse_scheme(scheme)
+    tile = dict(BM=TOKENS_4BIT, BN=CHANNELS, STAGE=STAGES_4BIT) if w == 4 else dict(BM=TOKENS, BN=CHANNELS, STAGE=STAGES)
     if a >= 16 and w >= 16:
-        return TileConfig(BK=64, MMA="TCGEN05_F16_F32")
+        return TileConfig(**tile, BK=64, MMA="TCGEN05_F16_F32")
     if a < 16:
         q = QConfig(QBITS=w, GSIZE=g, SYM=sym, PACK_DIM="PackDim::K")
         qa = QConfig(QBITS=a, GSIZE=g, SYM=sym, PACK_DIM="PackDim::K")
-        return TileConfig(BK=128, MMA="TCGEN05_S8_S32", QCFGA=qa, QCFGB=q)
-    return TileConfig(BK=64, MMA="TCGEN05_F16_F32",
+        return TileConfig(**tile, BK=128, MMA="TCGEN05_S8_S32", QCFGA=qa, QCFGB=q)
+    return TileConfig(**tile, BK=64, MMA="TCGEN05_F16_F32",
                       QCFGB=QConfig(QBITS=w, GSIZE=g, SYM=sym, PACK_DIM="PackDim::MN"))
 
 
 def get_best_tile_configs(batch_range: int, strategy_list: list[str]) -> dict:
     """B200 counterpart of the solver's hard-coded shortlist (bits_solver.py:425-515): the candidate tiles per scheme
-    for a batch range.  The sm_100a kernel has one tile per scheme whatever the batch (its token tile adapts to the
-    rows an expert has: up to 176, in steps of 16), so every batch range maps to the same single candidate."""
+    for a batch range.  The sm_100a kernel has one tile per scheme (its token tile adapts to the rows an expert has, in
+    steps of 32; a batch whose experts all have few rows runs 32-row tiles), so every batch range maps to the same
+    single candidate."""
     return {s: [b200_tile(s)] for s in strategy_list}
 
 
@@ -105,17 +114,18 @@ def profile(schemes=None, shapes=((2816, 2048), (2048, 1408)), iters: int = 20) 
     from . import gg, _lib
     from .weights import parse_scheme, SCHEMES, EXTRA_SCHEMES
     dev = torch.device("cuda", torch.cuda.current_device())
-    sms = _lib.lib().mxmoe_device_sm_count()
+    pairs = _lib.lib().mxmoe_device_sm_count() // 2
     table = {}
     for scheme in (schemes or SCHEMES + EXTRA_SCHEMES):
         a_bits, w_bits, g, sym = parse_scheme(scheme)
+        tile = b200_tile(scheme)
         entry = {"inc_by_nk": {}}
         for (N, K) in shapes:
-            nt = (N + 127) // 128
+            nt = -(-N // tile.BN)
             pts_t, pts_ms = [], []
             for waves in (0.5, 1, 2, 3, 4, 6, 8, 12, 16):
-                m_tiles = max(1, round(waves * sms / nt))
-                M = m_tiles * 176
+                m_tiles = max(1, round(waves * pairs / nt))
+                M = m_tiles * tile.BM
                 expanded = a_bits == 4          # the layer's activation format for w4a4: one byte 16*q per code
                 A = (torch.randint(-30000, 30000, (M, K * (8 if expanded else a_bits) // 16), dtype=torch.int16, device=dev)
                      if a_bits < 16 else torch.randn(M, K, device=dev).half())

@@ -162,12 +162,24 @@ def test_perf_table_schema_matches_the_solver_input():
         sk = "1" if ("a16" in scheme or scheme == "fp16") else "3"
         assert list(by_key) == [sk]
         key = repr(perf_table.b200_tile(scheme))
-        assert key.startswith("TileConfig(BM=176, BN=128, BK=") and key in by_key[sk]
+        assert key in by_key[sk]
         cost = by_key[sk][key]
         assert {"first_iter_cost", "inc", "stderr"} <= set(cost) and cost["inc"] > 0
-    # int8 tiles must be cheaper than fp16 tiles of the same shape, 4-bit weight-only the most expensive
-    inc = {s: next(iter(next(iter(v.values())).values()))["inc"] for s, v in table.items()}
+    # per token row of a tile int8 must be cheaper than fp16, 4-bit weight-only the most expensive
+    inc = {s: next(iter(next(iter(v.values())).values()))["inc"] / perf_table.b200_tile(s).BM for s, v in table.items()}
     assert inc["w8a8_g-1_sym"] < inc["fp16"] < inc["w4a16_g128_asym"]
+
+
+def test_perf_table_tiles_are_those_of_the_default_kernel():
+    from mxmoe_b200 import perf_table
+    csrc = os.path.join(ROOT, "mxmoe_b200", "csrc")
+    types, duo = (open(os.path.join(csrc, f)).read() for f in ("gg_types.h", "gg_duo_kernel.cu"))
+    tok, tok4 = map(int, re.search(r"kDuoTok = (\d+), kDuoTokCvt = (\d+),", types).groups())
+    stages4, stages = map(int, re.search(r"kStages\s*= kShort \? \d+ : \(kMode \? (\d+) : (\d+)\);", duo).groups())
+    channels = 2 * int(re.search(r"kWT = (\d+);", types).group(1))
+    for scheme in weights.SCHEMES + weights.EXTRA_SCHEMES:
+        t = perf_table.b200_tile(scheme)
+        assert (t.BM, t.BN, t.STAGE) == ((tok4, channels, stages4) if scheme.startswith("w4") else (tok, channels, stages))
 
 
 def test_verify_decodes_the_stored_layouts():
