@@ -327,7 +327,7 @@ def roofline_of(layer, spec, counts, d1, d2, peaks):
     achieved = flops_launch / (gemm_ms * 1e-3) / 1e12
     bytes_launch = byts / 2
     return {
-        "bound": "tensor", "kernel": "gg_swap_kernel", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
+        "bound": "tensor", "kernel": "gg_duo_kernel", "achieved": achieved, "peak": peak, "unit": "TFLOP/s",
         "frac": achieved / peak, "traffic": ncu_traffic(spec.name),
         "peak_source": (f"{peaks['source']} cuBLAS bf16 burst, x2 for the {share_i8:.0%} of the flops that run as "
                         "tcgen05 kind::i8 (twice the bf16 issue rate)"),

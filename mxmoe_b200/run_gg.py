@@ -110,7 +110,7 @@ def bench(input_path: str, output_prefix: str | None, layer: str | None = None, 
                 tf = flops / (ms * 1e-3) / 1e12
                 base_ms = ms if kind == "fp16" else base_ms
                 schemes = sorted({scheme_name(p["a_bits"], p["w_bits"], p["gsize"], p["sym"]) for p in probs})
-                name = "gg_swap_kernel[fp16]" if kind == "fp16" else f"gg_swap_kernel[{', '.join(schemes)}]"
+                name = "gg_duo_kernel[fp16]" if kind == "fp16" else f"gg_duo_kernel[{', '.join(schemes)}]"
                 rows.append((name, ms, tf, base_ms / ms))
                 del g
             results[(lid, blk)] = rows

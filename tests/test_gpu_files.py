@@ -20,7 +20,7 @@ def test_bench_reads_workload_json_and_writes_reference_csv(cuda_device, tmp_pat
         with open(tmp_path / "out" / f"bench-7-{blk}.csv") as f:
             rows = list(csv.reader(f))
         assert rows[0] == ["kernel_name", "avg_time", "TFLOPS", "speedup"]      # test.cu:858
-        assert len(rows) == 3 and rows[1][0] == "gg_swap_kernel[fp16]" and float(rows[1][3]) == 1.0
+        assert len(rows) == 3 and rows[1][0] == "gg_duo_kernel[fp16]" and float(rows[1][3]) == 1.0
         assert float(rows[2][1]) > 0 and float(rows[2][2]) > 0
 
 
