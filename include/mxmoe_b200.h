@@ -112,12 +112,14 @@ size_t mxmoe_gg_workspace_bytes(int problem_count);
 typedef struct mxmoe_gg_plan {
   int32_t count;     /* problems kept (empty ones are dropped) */
   int32_t needs_cvt; /* kernel variant: 0 no 4-bit operand, 1 4-bit weights only, 2 packed 4-bit activations too */
-  int32_t flags;     /* bit 0: a problem redirects its C rows (c_row0_dev) or uses w4a16_g-1_asym: only the SWAP kernel can run it;
+  int32_t flags;     /* bit 0: a problem redirects its C rows (c_row0_dev, c_row_ptrs), has out_mode 2 or uses w4a16_g-1_asym:
+                               only the SWAP and SWAP2 kernels can run it;
+                        bit 1: SWAP2 with token tiles of 32 rows and a ring of 10 stages (set by prepare when no problem has
+                               more than 32 rows; the caller may set or clear it before mxmoe_gg_run, e.g. set it when
+                               the row counts come from device memory and are known to be small on average; the other
+                               kernels have one geometry and ignore it);
                         bit 2: a problem uses an optional result form (out_mode 2, c_row0_dev, c_row_ptrs): the launch runs the
-                               kernel instance that has them, the weight tensor maps have rank 4;
-                        bit 1: SWAP kernel with token tiles of 32 rows and a ring of 10 stages, 7 of two K blocks with 4-bit weights (set by prepare when no
-                        problem has more than 32 rows; the caller may set or clear it before mxmoe_gg_run, e.g. set
-                        it when the row counts come from device memory and are known to be small on average) */
+                               kernel instance that has them, the weight tensor maps have rank 4 */
   int32_t kernel;    /* the kernel mxmoe_gg_run launches (an mxmoe_gg_kernel value): chosen by mxmoe_gg_prepare from the
                         environment variable MXMOE_GG_KERNEL (swap2 | swap | single | pair; default swap2) */
 } mxmoe_gg_plan;
@@ -157,7 +159,7 @@ int mxmoe_gg_launch(const mxmoe_gg_problem* problems, int problem_count, void* w
  * so that the workspace can be launched again. */
 int mxmoe_gg_check(void* workspace, void* stream);
 
-/* Test hook for the bounded waits of the kernel with swapped operands (no counterpart in the reference, whose
+/* Test hook for the bounded waits of the kernels with swapped operands, SWAP and SWAP2 (no counterpart in the reference, whose
  * kernels cannot time out).  `timeout_ms` > 0 replaces the 1000 ms limit of every device-side wait of later
  * launches over `workspace`; `skip_stage` >= 0 makes the producer of CTA 0 announce more weight bytes than it
  * loads for that pipeline stage (counted from the start of its work), so that the wait for them runs out: the launch then ends

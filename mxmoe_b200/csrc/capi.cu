@@ -234,7 +234,7 @@ int build_problem(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, mxb::GG
 }
 
 // The same problem for the kernel with swapped operands: tensor maps with its boxes (weights: 128 channels per
-// box; activations: 176-row and 32-row boxes).  `d` has been validated by build_problem already.
+// box; activations: boxes of 176 rows, of 32, and of half a CTA pair's token tile).  `d` has been validated by build_problem already.
 // `ext`: the launch runs the kernel instance with the optional result forms; its weight maps have rank 4
 int build_problem_swap(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, const mxb::GGProblemDev& d,
                        mxb::GGSwapProblemDev* o, bool bulk_everywhere, bool ext, int half_rows) {
@@ -270,8 +270,8 @@ int build_problem_swap(EncodeTiledFn enc, const mxmoe_gg_problem& p, int idx, co
     if ((rc = encode_2d(enc, &o->tmXs, p.A, f16, 2, K, a_rows, 64, mxb::kXBoxSmall, s128, "A", idx, lda))) return rc;
     if ((rc = encode_2d(enc, &o->tmXh, p.A, f16, 2, K, a_rows, 64, half_rows, s128, "A", idx, lda))) return rc;
   } else if (d.scheme == mxb::SCH_W4A4) {
-    // packed rows: 64 bytes of K per stage, unswizzled (the converters expand them in shared memory); token tiles
-    // of such launches have at most 128 rows, loaded as 32-row boxes
+    // packed rows: 64 bytes of K per stage, unswizzled (the converters expand them in shared memory), loaded as 32-row
+    // boxes: a single CTA's tile of such a problem has at most 128 rows, a pair's 192, half of them per CTA
     if ((rc = encode_2d(enc, &o->tmXs, p.A, u8, 1, K / 2, a_rows, 64, mxb::kXBoxSmall, CU_TENSOR_MAP_SWIZZLE_NONE, "A", idx, lda))) return rc;
     o->tmX = o->tmXs;
     o->tmXh = o->tmXs;
@@ -309,7 +309,7 @@ int default_kernel() {
   return GGK_SWAP2;
 }
 
-// token-tile geometry of the CTA-pair kernel: chosen from the row counts unless MXMOE_GG_TILES = small | large overrides
+// token-tile geometry of the SWAP2 kernel (the others have one each): chosen from the row counts unless MXMOE_GG_TILES = small | large overrides
 // it (read when a workspace is prepared)
 bool small_tiles_at_prepare(bool few_rows) {
   const char* e = getenv("MXMOE_GG_TILES");
@@ -381,7 +381,7 @@ int mxmoe_gg_prepare(const mxmoe_gg_problem* problems, int problem_count, void* 
     if (rc) return rc;
     rc = build_problem_swap(st->encode, problems[i], i, dev[kept], &swp[kept], bulk_everywhere, ext, half_rows);
     if (rc) return rc;
-    // redirected C rows and the per-channel 4-bit weight-only scheme exist in the SWAP kernel only
+    // redirected C rows, the fused silu and the per-channel 4-bit weight-only scheme exist in the SWAP and SWAP2 kernels only
     if (problems[i].c_row0_dev || problems[i].c_row_ptrs || (dev[kept].scheme == mxb::SCH_W4A16G128 && problems[i].q.gsize == -1) ||
         problems[i].out_mode == mxb::OUT_SILU) redirect = true;
     if (problems[i].M > max_rows) max_rows = problems[i].M;

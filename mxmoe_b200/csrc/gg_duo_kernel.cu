@@ -28,7 +28,8 @@
 //   4-11    epilogue, two warps per TMEM lane quarter, alternating 32-token chunks; scales and problem fields are loaded
 //           one tile ahead (loading them per tile cost w8a8 8 x [4096, 2048, 1408] 20 us of 94)
 //   12-23   converters in three groups of four warps that take converted K blocks in turn (two groups: packed w4a4 and
-//           w4a16 5-8 % slower; four groups have 72 registers per thread and spill, which costs more than they bring)
+//           w4a16 5-8 % slower; four groups have 72 registers per thread and spill more than the 2-5 words of
+//           the long-tile instances at 80, which costs more than they bring)
 //
 // Barriers.  full[s] (leader): everything the MMAs of stage s read is in place in both CTAs - the loads of both (the
 // cta_group::2 form of a load completes on the leader's barrier) and, for converted weights, eight arrivals of converter
@@ -646,7 +647,8 @@ gg_duo_kernel(const GGSwapProblemDev* __restrict__ problems, int count, GGStatus
     // instructions is what bounds launches with 4-bit weights, so nothing is walked or divided per block.
     int stage0 = 0, wbar0 = 0, slot0 = 0, turn = 0;
     uint32_t wphase0 = 0, it0 = 0;
-    uint32_t i1 = -64, i2 = -64, i3 = -64, i4 = -64;   // stage counts of the last four converted K blocks before the tile (none: long ago)
+    constexpr uint32_t kLongAgo = 0u - 64u;
+    uint32_t i1 = kLongAgo, i2 = kLongAgo, i3 = kLongAgo, i4 = kLongAgo;   // stage counts of the last four converted K blocks before the tile (none: long ago)
     bool ok = true;
     TileRec nrec = tile_rec(0);
     for (int i = 0; ok && i < my_tiles; ++i) {

@@ -10,7 +10,7 @@ constexpr int kWSlotBytes  = kWT * kRowBytes;   // 16 KiB: plain weights, or 8 /
 constexpr int kEpiStageS   = 2048;              // per epilogue warp: 16 token pairs x 32 channels x 4 bytes
 constexpr uint32_t kASlotCols = 32;             // TMEM columns of one converted K block (128 bytes of K per channel)
 constexpr int kCvtGroup    = 4;                 // warps per converter group (one per TMEM lane quarter)
-constexpr int kEpiWarps    = 8;                 // two per TMEM lane quarter (warps 2-5 and 7-10)
+constexpr int kEpiWarps    = 8;                 // two per TMEM lane quarter
 
 // What every role needs to know about one tile, precomputed once per CTA: looking a tile up in the
 // scheduling tables is a chain of dependent shared-memory loads, each of which takes hundreds of cycles
@@ -18,10 +18,10 @@ constexpr int kEpiWarps    = 8;                 // two per TMEM lane quarter (wa
 struct TileRec {
   int pk;       // problem | scheme << 8 | k-blocks << 12
   int x_row;    // buffer row of the tile's first token (A and scale_a)
-  int nt;       // channel tile | tokens in the tile (1 .. kTT) << 16
+  int nt;       // channel tile | tokens in the tile (1 .. the kernel's longest) << 16
   int c_row;    // row of C of the tile's first token
 };
-constexpr int kMaxRecs = 512;   // tiles per CTA kept in the table; later ones are looked up on the fly
+constexpr int kMaxRecs = 512;   // tiles per CTA kept in the single-CTA kernel's table; later ones are looked up on the fly
 
 struct TileS {
   int p, scheme, nkb, x_row, n_tile, ntok, c_row;
@@ -76,8 +76,7 @@ __device__ __forceinline__ TileS decode_rec(const TileRec& r) {
   return t;
 }
 
-// named barriers (ids in Geo): stage s is ready (watcher and the stage's converter group -> MMA warp);
-// accumulator b is drained (epilogue warps -> MMA warp)
+// named barriers (the single-CTA kernel's ids are in its Geo, the CTA-pair kernel uses them in the epilogue only)
 __device__ __forceinline__ void nbar_sync(int id, int nthreads) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }

@@ -51,10 +51,10 @@ struct alignas(128) GGProblemDev {
 };
 static_assert(sizeof(GGProblemDev) == 384, "GGProblemDev layout");
 
-// The same problem as seen by the kernel with swapped operands (gg_swap_kernel.cu): the weights are the
-// M side of the MMA (tiles of 128 output channels), the tokens the N side (tiles of up to 176 rows).
+// The same problem as seen by the kernels with swapped operands (gg_duo_kernel.cu, gg_swap_kernel.cu): the weights are the
+// M side of the MMA (128 output channels per CTA), the tokens the N side.
 constexpr int kWT = 128;   // output channels per tile (tcgen05 M)
-constexpr int kTT = 176;   // tokens per tile (tcgen05 N, any multiple of 16 up to this)
+constexpr int kTT = 176;   // tokens per tile on single CTAs (tcgen05 N, any multiple of 16 up to this)
 // the kernel on CTA pairs (gg_duo_kernel.cu): tokens per tile without / with 4-bit weights in the launch
 constexpr int kDuoTok = 256, kDuoTokCvt = 192, kDuoTokShort = 32;   // (short: launches with few rows per problem)
 constexpr int kXBoxSmall = 32;   // rows of the small activation box (short token tiles load only what they need)
@@ -89,7 +89,7 @@ struct alignas(256) GGStatus {
   // tiles and the stages
   unsigned long long prof[16];
   int prof_on;      // per-role cycle counters wanted (costs a few percent)
-  int timeout_ms;   // limit of every bounded wait of the kernel with swapped operands; 0 = 1000 ms
+  int timeout_ms;   // limit of every bounded wait of the kernels with swapped operands; 0 = 1000 ms
   int skip_stage;   // test hook: 1 + the pipeline stage (counted from the start of CTA 0's work) for which CTA 0's
                     // producer announces more weight bytes than it loads, so that the wait for them runs out; 0 = none
   int pad[25];
