@@ -1,4 +1,5 @@
-// Persistent mixed-precision grouped GEMM for sm_100a on CTA PAIRS (tcgen05 cta_group::2): the kernel of every launch.
+// Persistent mixed-precision grouped GEMM for sm_100a on CTA PAIRS (tcgen05 cta_group::2): the default of every launch of
+// two CTAs or more.
 //
 // Same contract and operand roles as gg_swap_kernel.cu (one launch walks a device-side list of problems
 // C[M,N] = A[M,K] x B[N,K]^T, each with its own scheme; reference: mxmoe/kernels/compose_kernel.py:150-295,
